@@ -13,9 +13,9 @@
 //   src/atari.rs:584-614  run_frame / run_one_cycle
 //   src/headless_tia.rs   HeadlessTia
 //   src/pia.rs            Pia
-// The instruction decoder is organised by the 6502 opcode bit fields
-// (aaa bbb cc) instead of one 151-way switch: lanes executing different
-// opcodes that share an addressing mode or an ALU operation share code.
+// The interpreter (Emu::run) is driven by a table of eight words per opcode
+// instead of a switch: most instructions run through one straight sequence of
+// selects, so lanes at different opcodes share it too.
 #pragma once
 #include <stdint.h>
 
@@ -23,6 +23,11 @@
 #include "fa_layout.h"
 
 namespace fa {
+
+// Instructions after which a converged group checks, at its next branch, that
+// its lanes are still together (they check at once where a branch parts them,
+// and after returns, indirect jumps and interrupts).
+constexpr uint32_t FA_BURST = 32;
 
 enum : uint32_t { F_C = 1, F_Z = 2, F_I = 4, F_D = 8, F_B = 16, F_U = 32, F_V = 64, F_N = 128 };
 
@@ -42,14 +47,270 @@ static __constant__ uint32_t c_action_table[18] = {
     act_word(0, 1, 0, 1, 1), act_word(0, 1, 1, 0, 1),
 };
 
-// Bit op of word op>>5 is set for the 151 legal opcodes (src/cpu.rs:253-1141).
-static __constant__ uint32_t c_legal[8] = {
-    0x63636763u, 0x63637773u, 0x63637763u, 0x63637763u,
-    0x27737572u, 0x77737777u, 0x63637773u, 0x63637773u,
+// ---------------------------------------------------------------- opcode table
+// What an opcode does, as eight words.  Emu::run executes most instructions
+// from them without a branch: registers, operands, flags and destination are
+// selected by byte permutes whose selectors are the words' low halves (so no
+// field is extracted for them).  Lanes at different opcodes share its code too.
+struct alignas(16) OpWord {
+    uint32_t ix;   // over (registers, $80, 0): the index; high half: T_*
+    uint32_t rs;   // over (registers, 0): the register operand; high half: cycles without the page-crossing and branch penalties
+    uint32_t rd;   // over (registers, result): the new registers; high half: bytes
+    uint32_t bs;   // over (operand bytes): the base address; high half: m of Emu::alu
+    uint32_t qs;   // over (flags, 1, $FF, 0): what is added; high half: OP_* | T_IND, T_INDY, T_K
+    uint32_t fs;   // over (flags, result and its flags): the new flags
+    uint32_t am;   // address mask, $FF (wraps in zero page) or $FFFF; high half: what the operand is XORed with.  Branches: the flag tested
+    uint32_t xs;   // over (memory operand, first operand byte): the operand
 };
+enum : uint32_t {                                                     // in ix
+    T_CTRL = 1u << 16,    // not the straight path: branch, stack or jump; with T_MEM: through a zero-page pointer
+    T_MEM = 1u << 17,     // has a memory operand
+    T_WR = 1u << 31,      // writes it (stores, read-modify-write); the sign bit: run() clears ROM addresses' with it
+    T_FIX = 1u << 20,     // the fix-up read of an indexed access is always made
+    T_UV = 1u << 23,      // sets V; decimal mode applies (ADC, SBC)
+    T_BR = 1u << 24,      // branch, taken when the flag is clear (T_BI) or set
+    T_BI = 1u << 27,
+    T_CTL = 1u << 28,     // may leave lanes of a converged group at different pcs
+    T_ODD = 1u << 29,     // shifts, BIT, operations on I, D and V
+};
+// With the operation: through a zero-page pointer, (zp),Y; the XOR term of Emu::alu kept (all but AND).
+enum : uint32_t { T_IND = 0x40u, T_INDY = 0x80u, T_K = 0x8000u };
+enum : uint32_t {
+    // on a value read (memory or immediate)
+    OP_ORA, OP_AND, OP_EOR, OP_ADC, OP_LDA, OP_CMP, OP_SBC, OP_LDX, OP_LDY, OP_CPX, OP_CPY, OP_BIT,
+    // on a value read, written back
+    OP_ASL, OP_ROL, OP_LSR, OP_ROR, OP_DEC, OP_INC,
+    // stores
+    OP_STA, OP_STX, OP_STY,
+    // no operand
+    OP_CLC, OP_SEC, OP_CLI, OP_SEI, OP_CLV, OP_CLD, OP_SED, OP_TAX, OP_TXA, OP_TAY, OP_TYA, OP_TSX, OP_TXS,
+    OP_INX, OP_INY, OP_DEX, OP_DEY, OP_NOP,
+    // branches, in opcode order
+    OP_BPL, OP_BMI, OP_BVC, OP_BVS, OP_BCC, OP_BCS, OP_BNE, OP_BEQ,
+    // stack and control
+    OP_PHP, OP_PHA, OP_JSR, OP_BRK, OP_PLP, OP_PLA, OP_RTS, OP_RTI, OP_JMP, OP_JMPI,
+    OP_ILL
+};
+struct OpTable { OpWord e[256]; };
+// The 151 legal opcodes of src/cpu.rs:253-1141; the rest are OP_ILL.
+constexpr OpTable make_op_table()
+{
+    OpTable t{};
+    constexpr uint32_t A = 0, X = 1, Y = 2, S = 3, N = 4;            // registers; N: none
+    constexpr uint32_t QC = 2, Q1 = 4, QF = 5, Q0 = 6;               // what is added: carry, 1, $FF, 0
+    constexpr uint32_t ZP = 1, AB = 2, IM = 3, NO = 0;               // operand: zero page, absolute, immediate, none
+    for (uint32_t op = 0; op < 256u; op++)
+        t.e[op] = OpWord{ 0x5554u | T_CTRL | T_CTL, 0x4444u, 0x3210u | (1u << 16), 0x1111u, 0x6666u | (OP_ILL << 16), 0x3210u,
+                          0xFFu, 0x1111u };
+    auto set = [&](uint32_t op, uint32_t o, uint32_t mode, uint32_t idx, uint32_t flags, uint32_t ind, uint32_t len,
+                   uint32_t cyc) {
+        uint32_t src = N, dst = N, q = Q0, b = 0, m = 1, f = 0, kx = T_K;
+        bool nz = true, c = false, v = false, use = true;            // use: the operand enters the result
+        switch (o) {
+        case OP_ORA: src = dst = A; break;
+        case OP_AND: src = dst = A; kx = 0; break;
+        case OP_EOR: src = dst = A; m = 0; break;
+        case OP_LDA: dst = A; break;
+        case OP_LDX: dst = X; break;
+        case OP_LDY: dst = Y; break;
+        case OP_ADC: src = dst = A; m = 2; q = QC; c = v = true; f |= T_UV; break;
+        case OP_SBC: src = dst = A; m = 2; q = QC; b = 0xFF; c = v = true; f |= T_UV; break;
+        case OP_CMP: src = A; m = 2; q = Q1; b = 0xFF; c = true; break;
+        case OP_CPX: src = X; m = 2; q = Q1; b = 0xFF; c = true; break;
+        case OP_CPY: src = Y; m = 2; q = Q1; b = 0xFF; c = true; break;
+        case OP_ASL: case OP_LSR: f |= T_ODD | (mode ? T_WR : 0u); break;
+        case OP_ROL: case OP_ROR: q = QC; f |= T_ODD | (mode ? T_WR : 0u); break;
+        case OP_INC: q = Q1; f |= T_WR; break;
+        case OP_DEC: q = QF; f |= T_WR; break;
+        case OP_STA: src = A; f |= T_WR; nz = use = false; break;
+        case OP_STX: src = X; f |= T_WR; nz = use = false; break;
+        case OP_STY: src = Y; f |= T_WR; nz = use = false; break;
+        case OP_CLC: c = true; nz = false; break;
+        case OP_SEC: b = 0x100; c = true; nz = false; break;
+        case OP_TAX: src = A; dst = X; break;
+        case OP_TXA: src = X; dst = A; break;
+        case OP_TAY: src = A; dst = Y; break;
+        case OP_TYA: src = Y; dst = A; break;
+        case OP_TSX: src = S; dst = X; break;
+        case OP_TXS: src = X; dst = S; nz = false; break;
+        case OP_INX: src = dst = X; q = Q1; break;
+        case OP_INY: src = dst = Y; q = Q1; break;
+        case OP_DEX: src = dst = X; q = QF; break;
+        case OP_DEY: src = dst = Y; q = QF; break;
+        case OP_NOP: nz = false; break;
+        case OP_BIT: case OP_CLI: case OP_SEI: case OP_CLV: case OP_CLD: case OP_SED: f |= T_ODD; nz = false; break;
+        default: f |= T_CTRL; nz = false; break;
+        }
+        const bool mem = mode == ZP || mode == AB;
+        if (mem) f |= T_MEM;
+        if (ind) f |= T_CTRL;
+        // Without a memory operand the address is $80: RAM, read and not used.
+        const uint32_t i = !mem ? 4u : idx == N ? 5u : idx;
+        const uint32_t d = dst == N ? 0x3210u : (0x3210u & ~(0xFu << (4u * dst))) | (4u << (4u * dst));
+        const uint32_t fl = (nz ? 0x74u : 0x10u) | (c ? 0x500u : 0x200u) | (v ? 0x6000u : 0x3000u);
+        t.e[op] = OpWord{ 0x5550u | i | f | flags, 0x4440u | src | (cyc << 16), d | (len << 16),
+                          (mode == ZP ? 0x1110u : mode == AB ? 0x1140u : 0x1111u) | (m << 16), 0x6660u | q | ((o | ind | kx) << 16), fl,
+                          (mode == AB ? 0xFFFFu : 0xFFu) | (b << 16),
+                          !use ? 0x1111u : mem ? 0x1110u : mode == IM ? 0x1114u : 0x1111u };
+    };
+    // cc = 01: eight operations, eight modes.
+    const uint32_t g1[8] = { OP_ORA, OP_AND, OP_EOR, OP_ADC, OP_STA, OP_LDA, OP_CMP, OP_SBC };
+    for (uint32_t k = 0; k < 8u; k++) {
+        const uint32_t b = (k << 5) | 1u, o = g1[k];
+        const bool st = o == OP_STA;
+        const uint32_t fix = st ? T_FIX : 0u, e = st ? 1u : 0u;
+        set(b | 0x00u, o, AB, N, 0, T_IND, 2, 6);                                  // (zp,X)
+        set(b | 0x04u, o, ZP, N, 0, 0, 2, 3);                                      // zp
+        if (!st) set(b | 0x08u, o, IM, N, 0, 0, 2, 2);                             // #imm
+        set(b | 0x0Cu, o, AB, N, 0, 0, 3, 4);                                      // abs
+        set(b | 0x10u, o, AB, Y, fix, T_IND | T_INDY, 2, 5 + e);                   // (zp),Y
+        set(b | 0x14u, o, ZP, X, 0, 0, 2, 4);                                      // zp,X
+        set(b | 0x18u, o, AB, Y, fix, 0, 3, 4 + e);                                // abs,Y
+        set(b | 0x1Cu, o, AB, X, fix, 0, 3, 4 + e);                                // abs,X
+    }
+    // cc = 10: shifts, INC, DEC; LDX, STX.
+    const uint32_t g2[8] = { OP_ASL, OP_ROL, OP_LSR, OP_ROR, OP_STX, OP_LDX, OP_DEC, OP_INC };
+    for (uint32_t k = 0; k < 8u; k++) {
+        const uint32_t b = (k << 5) | 2u, o = g2[k];
+        if (o == OP_STX || o == OP_LDX) {
+            set(b | 0x04u, o, ZP, N, 0, 0, 2, 3);
+            set(b | 0x0Cu, o, AB, N, 0, 0, 3, 4);
+            set(b | 0x14u, o, ZP, Y, 0, 0, 2, 4);
+            if (o == OP_LDX) {
+                set(b | 0x00u, o, IM, N, 0, 0, 2, 2);
+                set(b | 0x1Cu, o, AB, Y, 0, 0, 3, 4);
+            }
+            continue;
+        }
+        set(b | 0x04u, o, ZP, N, 0, 0, 2, 5);
+        set(b | 0x0Cu, o, AB, N, 0, 0, 3, 6);
+        set(b | 0x14u, o, ZP, X, 0, 0, 2, 6);
+        set(b | 0x1Cu, o, AB, X, T_FIX, 0, 3, 7);
+        if (k < 4u) set(b | 0x08u, o, NO, N, 0, 0, 1, 2);                          // of A
+    }
+    // cc = 00: BIT, STY, LDY, CPY, CPX.
+    set(0x24, OP_BIT, ZP, N, 0, 0, 2, 3); set(0x2C, OP_BIT, AB, N, 0, 0, 3, 4);
+    set(0x84, OP_STY, ZP, N, 0, 0, 2, 3); set(0x8C, OP_STY, AB, N, 0, 0, 3, 4); set(0x94, OP_STY, ZP, X, 0, 0, 2, 4);
+    set(0xA0, OP_LDY, IM, N, 0, 0, 2, 2); set(0xA4, OP_LDY, ZP, N, 0, 0, 2, 3); set(0xAC, OP_LDY, AB, N, 0, 0, 3, 4);
+    set(0xB4, OP_LDY, ZP, X, 0, 0, 2, 4); set(0xBC, OP_LDY, AB, X, 0, 0, 3, 4);
+    set(0xC0, OP_CPY, IM, N, 0, 0, 2, 2); set(0xC4, OP_CPY, ZP, N, 0, 0, 2, 3); set(0xCC, OP_CPY, AB, N, 0, 0, 3, 4);
+    set(0xE0, OP_CPX, IM, N, 0, 0, 2, 2); set(0xE4, OP_CPX, ZP, N, 0, 0, 2, 3); set(0xEC, OP_CPX, AB, N, 0, 0, 3, 4);
+    // Implied.
+    const uint32_t imp[18][2] = { { 0x18, OP_CLC }, { 0x38, OP_SEC }, { 0x58, OP_CLI }, { 0x78, OP_SEI }, { 0xB8, OP_CLV },
+                                  { 0xD8, OP_CLD }, { 0xF8, OP_SED }, { 0xAA, OP_TAX }, { 0x8A, OP_TXA }, { 0xA8, OP_TAY },
+                                  { 0x98, OP_TYA }, { 0xBA, OP_TSX }, { 0x9A, OP_TXS }, { 0xE8, OP_INX }, { 0xC8, OP_INY },
+                                  { 0xCA, OP_DEX }, { 0x88, OP_DEY }, { 0xEA, OP_NOP } };
+    for (uint32_t k = 0; k < 18u; k++) set(imp[k][0], imp[k][1], NO, N, 0, 0, 1, 2);
+    // Branches by opcode bits 6-7 (N, V, C, Z) and 5 (clear, set); F holds Z as a byte that is 0 when Z is set.
+    for (uint32_t k = 0; k < 8u; k++) {
+        const uint32_t fl = k >> 1, on = k & 1u;
+        set(0x10u | (k << 5), OP_BPL + k, NO, N, T_CTL | T_BR | (((fl == 3u) ? on : !on) ? T_BI : 0u), 0, 2, 2);
+        t.e[0x10u | (k << 5)].am = fl == 0u ? 0x8080u : fl == 1u ? 0x80000000u : fl == 2u ? 0x10000u : 0xFFu;
+    }
+    // Stack, control.
+    set(0x08, OP_PHP, NO, N, 0, 0, 1, 3); set(0x48, OP_PHA, NO, N, 0, 0, 1, 3); set(0x28, OP_PLP, NO, N, 0, 0, 1, 4);
+    set(0x68, OP_PLA, NO, N, 0, 0, 1, 4); set(0x20, OP_JSR, NO, N, 0, 0, 2, 6); set(0x00, OP_BRK, NO, N, T_CTL, 0, 2, 7);
+    set(0x60, OP_RTS, NO, N, T_CTL, 0, 1, 6); set(0x40, OP_RTI, NO, N, T_CTL, 0, 1, 6); set(0x4C, OP_JMP, NO, N, 0, 0, 3, 3);
+    set(0x6C, OP_JMPI, NO, N, T_CTL, 0, 3, 5);
+    return t;
+}
+
+// Headless TIA registers whose write only stores bits of the value
+// (headless_tia.rs:225-298): private byte | shift << 8 | mask << 16; 0 for
+// the others.
+struct TiaTable { uint32_t w[64]; };
+constexpr TiaTable make_tia_table()
+{
+    TiaTable t{};
+    for (uint32_t r = 0; r < 64u; r++) t.w[r] = 0;
+    auto set = [&](uint32_t r, uint32_t o, uint32_t sh, uint32_t m) { t.w[r] = o | (sh << 8) | (m << 16); };
+    set(0x04, 164, 0, 0xFF); set(0x05, 165, 0, 0xFF);                 // NUSIZ
+    for (uint32_t k = 0; k < 4u; k++) set(0x06u + k, 166u + k, 0, 0xFF);   // COLUx
+    set(0x0A, 170, 0, 0xFF);                                          // CTRLPF
+    set(0x0B, 171, 3, 1); set(0x0C, 172, 3, 1);                       // REFP
+    for (uint32_t k = 0; k < 3u; k++) set(0x0Du + k, 173u + k, 0, 0xFF);   // PF
+    for (uint32_t k = 0; k < 3u; k++) set(0x1Du + k, 155u + k, 1, 1);      // ENAM0 ENAM1 ENABL
+    for (uint32_t k = 0; k < 5u; k++) set(0x20u + k, 146u + k, 0, 0xFF);   // HM
+    for (uint32_t k = 0; k < 3u; k++) set(0x25u + k, 159u + k, 0, 1);      // VDEL
+    set(0x28, 162, 1, 1); set(0x29, 163, 1, 1);                       // RESMP
+    return t;
+}
+
+// Bytes of shared memory by their 32-bit address there.  Pointers would do,
+// but the interpreter's loop selects between two of them and keeps several:
+// as generic pointers they cost 64-bit arithmetic.
+#ifdef __CUDA_ARCH__
+typedef uint32_t sptr;
+__device__ __forceinline__ sptr to_sptr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t lds8(sptr p)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts8(sptr p, uint32_t v)
+{
+    asm volatile("st.shared.u8 [%0], %1;" ::"r"(p), "r"(v) : "memory");
+}
+#else
+typedef uint8_t* sptr;
+__device__ __forceinline__ sptr to_sptr(const void* p) { return (uint8_t*)p; }
+__device__ __forceinline__ uint32_t lds8(const uint8_t* p) { return *p; }
+__device__ __forceinline__ void sts8(uint8_t* p, uint32_t v) { *p = (uint8_t)v; }
+#endif
+
+// The kernels copy the table into shared memory (load_op_table): a constant
+// load costs one pass per distinct index of the warp, a shared load does not.
+#ifdef __CUDACC__
+static __device__ const OpTable g_op = make_op_table();
+static __device__ const TiaTable g_tia = make_tia_table();
+__device__ __forceinline__ OpWord* op_table()
+{
+    __shared__ OpWord t[256];
+    return t;
+}
+__device__ __forceinline__ uint32_t* tia_table()
+{
+    __shared__ uint32_t t[64];
+    return t;
+}
+// Called by every thread of the CTA; a barrier must follow before the first
+// instruction.
+__device__ __forceinline__ void load_op_table()
+{
+    uint4* d = (uint4*)op_table();
+    const uint4* s = (const uint4*)g_op.e;
+    for (uint32_t k = threadIdx.x; k < 512u; k += blockDim.x) d[k] = s[k];
+    for (uint32_t k = threadIdx.x; k < 64u; k += blockDim.x) tia_table()[k] = g_tia.w[k];
+}
+#else
+inline const OpWord* op_table()
+{
+    static const OpTable t = make_op_table();
+    return t.e;
+}
+inline const uint32_t* tia_table()
+{
+    static const TiaTable t = make_tia_table();
+    return t.w;
+}
+#endif
+__device__ __forceinline__ OpWord ldw(sptr tab, uint32_t op)
+{
+#ifdef __CUDA_ARCH__
+    OpWord w;
+    const uint32_t a = tab + op * 32u;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.ix), "=r"(w.rs), "=r"(w.rd), "=r"(w.bs) : "r"(a));
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4 + 16];" : "=r"(w.qs), "=r"(w.fs), "=r"(w.am), "=r"(w.xs) : "r"(a));
+    return w;
+#else
+    return ((const OpWord*)tab)[op];
+#endif
+}
 
 // Packed TIA flag word (Emu::tw).
 enum : uint32_t { TW_WSYNC = 1u << 16, TW_FCOMP = 1u << 17, TW_PDUMP = 1u << 18,
+                  TW_CX = 1u << 23,      // headless only: a collision latch may be set (only an upload sets them)
                   // rendering console only
                   TW_HMOVE = 1u << 19, TW_LATCH = 1u << 20, TW_L4 = 1u << 21, TW_L5 = 1u << 22 };
 
@@ -73,7 +334,7 @@ __device__ __forceinline__ uint32_t cold_off(uint32_t o, uint32_t stride4) { ret
 // TIA or PIA register read (HeadlessTia::read, src/headless_tia.rs:205-223;
 // Pia::read I/O half, src/pia.rs:169-199), INTIM apart (pia_intim_io):
 // sel_uf carries the timer's underflow flag in bits 16 and up.
-static __device__ __noinline__ uint32_t io_read(uint32_t a, uint32_t pcnt, uint32_t pins, uint32_t pads,
+static __device__ __forceinline__ uint32_t io_read(uint32_t a, uint32_t pcnt, uint32_t pins, uint32_t pads,
                                          uint32_t ports, uint32_t sel_uf, const uint8_t* col, uint32_t stride4)
 {
     if (a & 0x80u) {                                                 // PIA: (a & 0x280) == 0x280
@@ -101,7 +362,7 @@ static __device__ __noinline__ uint32_t io_read(uint32_t a, uint32_t pcnt, uint3
 // HeadlessTia::write (src/headless_tia.rs:225-298).  tw is the packed flag
 // word, lw = scanline | paddle_counter<<16; both come back updated.  The
 // write-only registers live in the instance's HBM rows (col, stride4).
-static __device__ __noinline__ uint2 tia_write_io(uint32_t a, uint32_t v, uint32_t clock, uint32_t tw, uint32_t lw,
+static __device__ __forceinline__ uint2 tia_write_io(uint32_t a, uint32_t v, uint32_t clock, uint32_t tw, uint32_t lw,
                                            uint8_t* col, uint32_t stride4)
 {
     auto stp = [&](uint32_t o, uint32_t val) { col[cold_off(o, stride4)] = (uint8_t)val; };
@@ -681,7 +942,7 @@ static __device__ __noinline__ RRead render_io_read(uint32_t a, uint32_t owed, R
 // 2K of display data.  One out-of-line copy for every access site.
 static __device__ __forceinline__ uint32_t dpc_byte(uint32_t w, uint32_t k) { return (w >> ((k & 3u) * 8u)) & 0xFFu; }
 
-static __device__ __noinline__ uint32_t dpc_io(uint32_t a, uint32_t v, uint32_t wr, uint32_t* col, uint32_t S,
+static __device__ __forceinline__ uint32_t dpc_io(uint32_t a, uint32_t v, uint32_t wr, uint32_t* col, uint32_t S,
                                                const uint8_t* disp, uint32_t cyc_acc)
 {
     const uint32_t misc = col[(size_t)R_DPC_MISC * S];
@@ -820,7 +1081,7 @@ static __device__ __forceinline__ uint2 pia_now_of(uint32_t tv, uint32_t ps, uin
 // An INTIM read (pia.rs:187-190): the counted cycles settled, the underflow
 // flag cleared (tv = 0 with a prescaler left may gain a window by it).
 // Packed (tv | ps << 16, sel | uf << 16, tlim); the value read is tv & 0xFF.
-static __device__ __noinline__ uint4 pia_intim_io(uint32_t tv_ps, uint32_t sel_uf, uint32_t tlim)
+static __device__ __forceinline__ uint4 pia_intim_io(uint32_t tv_ps, uint32_t sel_uf, uint32_t tlim)
 {
     const uint32_t sel = sel_uf & 0xFFFFu;
     const uint2 t = pia_now_of(tv_ps & 0xFFFFu, tv_ps >> 16, sel, sel_uf >> 16, tlim);
@@ -831,7 +1092,7 @@ static __device__ __noinline__ uint4 pia_intim_io(uint32_t tv_ps, uint32_t sel_u
 // leaves the timer and its counting alone; a timer write replaces value,
 // prescaler, interval and flag, so the cycles counted so far no longer
 // matter.
-static __device__ __noinline__ uint4 pia_store_io(uint32_t a, uint32_t v, uint32_t ports, uint32_t tp, uint32_t su,
+static __device__ __forceinline__ uint4 pia_store_io(uint32_t a, uint32_t v, uint32_t ports, uint32_t tp, uint32_t su,
                                                   uint32_t tlim)
 {
     if (a & 0x10u) {
@@ -843,7 +1104,7 @@ static __device__ __noinline__ uint4 pia_store_io(uint32_t a, uint32_t v, uint32
 }
 // Packed (tv | ps << 16, sel | uf << 16, tlim) after settling and one exact
 // call of n cycles.
-static __device__ __noinline__ uint4 pia_sync_io(uint32_t tv_ps, uint32_t sel_uf, uint32_t tlim, uint32_t n)
+static __device__ __forceinline__ uint4 pia_sync_io(uint32_t tv_ps, uint32_t sel_uf, uint32_t tlim, uint32_t n)
 {
     const uint32_t sel = sel_uf & 0xFFFFu;
     uint32_t uf = sel_uf >> 16;
@@ -851,6 +1112,43 @@ static __device__ __noinline__ uint4 pia_sync_io(uint32_t tv_ps, uint32_t sel_uf
     uint32_t tv = t.x, ps = t.y;
     pia_tick_n(tv, ps, sel, uf, n);
     return make_uint4(tv | (ps << 16), sel | (uf << 16), pia_span_of(tv, ps, sel, uf), 0u);
+}
+
+// ---------------------------------------------------------------- decimal mode (cpu.rs:153-241)
+// ADC and SBC with D set: (a, nz, carry, V in bit 7) as Emu keeps them.
+static __device__ __forceinline__ uint4 decimal_op(bool sub, uint32_t a, uint32_t v, uint32_t c)
+{
+    if (sub) {
+        const uint32_t b = c ^ 1u;
+        const int bin = (int)a - (int)v - (int)b;
+        const uint32_t r = (uint32_t)bin & 0xFFu;
+        uint32_t lo = ((a & 0xFu) - (v & 0xFu) - b) & 0xFFu, lob = 0;
+        if (lo & 0x80u) { lo = (lo - 6u) & 0xFFu; lob = 1; }
+        uint32_t hi = ((a >> 4) - (v >> 4) - lob) & 0xFFu;
+        if (hi & 0x80u) hi = (hi - 6u) & 0xFFu;
+        return make_uint4(((hi & 0xFu) << 4) | (lo & 0xFu), r, bin >= 0 ? 1u : 0u, (a ^ v) & (a ^ r));
+    }
+    uint32_t lo = (a & 0xFu) + (v & 0xFu) + c;
+    if (lo > 9u) lo += 6u;
+    uint32_t hi = (a >> 4) + (v >> 4) + (lo > 0xFu ? 1u : 0u);
+    const uint32_t bin = (a + v + c) & 0xFFu, res = ((hi << 4) | (lo & 0xFu)) & 0xFFu;
+    const uint32_t nz = (bin ? 1u : 0u) | ((hi & 8u) << 12), vf = ~(a ^ v) & (a ^ res);
+    if (hi > 9u) hi += 6u;
+    return make_uint4(((hi & 0xFu) << 4) | (lo & 0xFu), nz, hi > 0xFu ? 1u : 0u, vf);
+}
+
+// The headless TIA's scanlines of a run of instruction ticks
+// (headless_tia.rs:153-198) that brought the beam from below 228 to `clk`
+// TIA clocks of the line it started on, no tick more than a line: what the
+// ticks one by one leave.  lw = scanline (below 262) | paddle_counter << 16.
+// Returns (clock, lw, tw).
+static __device__ __forceinline__ uint4 tia_fold_io(uint32_t clk, uint32_t lw, uint32_t tw)
+{
+    const uint32_t lines = clk / 228u;
+    uint32_t s = (lw & 0xFFFFu) + lines, pc = lw >> 16;
+    if (s >= 262u) { s %= 262u; tw |= TW_FCOMP; }
+    if (!(tw & TW_PDUMP) && pc < 256u) pc = pc + lines < 256u ? pc + lines : 256u;
+    return make_uint4(clk - lines * 228u, s | (pc << 16), tw & ~TW_WSYNC, 0u);
 }
 
 // SLICED: the core of E0 and 3F carts (with DPC, of DPC carts alone; with
@@ -869,11 +1167,24 @@ struct Emu {
     const uint8_t* rom;      // shared-memory ROM image, nbanks * 4 KiB
     uint32_t hot_lo, nbanks;
     // ---- CPU (src/cpu.rs:96-105)
-    uint32_t a, x, y, sp, p, pc;
-    uint32_t bank;           // bank index (bits 0-2) | hotspot accesses this frame << 3,
-                             // saturating at 511: the count is a scheduling key only
+    // P is kept apart: what an instruction sets costs one move or none, and
+    // PHP, BRK and the state rows assemble it (get_p / set_p).
+    uint32_t R, pc;          // a | x << 8 | y << 16 | sp << 24 (packed, so a table word selects the register)
+    uint32_t F;              // flags, by bytes: Z is set when byte 0 is 0; N is bit 7 of byte 0 or byte 1; C: byte 2
+                             // (0 or 1); V: bit 7 of byte 3
+    uint32_t p;              // P's I, B and unused bits
+    uint32_t pd;             // T_UV in decimal mode, else 0
+    uint32_t bank;           // 4K-bank carts: the bank's offset in the ROM image (index << 12)
+    uint32_t kb;             // scheduling key above pc: frame << 25 | hotspot accesses this frame << 16, each saturating
     uint32_t slices;         // SLICED (E0, 3F carts): the 1K ROM slice of window k in byte k
-    uint32_t cyc_acc;         // instruction cycles not yet added to Cpu::cycles in HBM
+    uint32_t cyc_acc;         // instruction cycles not yet added to Cpu::cycles in HBM (headless: up to the last sync)
+    // Headless time.  An instruction only adds its cycles to `el` and compares
+    // it with `dl`; the beam, the timer and the cycle counts are brought up to
+    // date (sync) when something reads or changes them, or when el reaches dl:
+    // the end of the timer's window, a frame limit, or an instruction that
+    // wrote WSYNC or VSYNC (dl = 0).
+    uint32_t el;             // cycles since the last sync
+    uint32_t dl;             // cycles from the last sync at which the frame loop must look
     // ---- PIA (src/pia.rs:26-44): timer unpacked, ports and input pins packed
     //      (touched only by I/O accesses)
     uint32_t tp;             // timer value | prescaler << 16 (the R_TIMER row word)
@@ -891,8 +1202,19 @@ struct Emu {
 
     // The instance's HBM rows.  Cpu::cycles, the frame counter and the run
     // status stay there and change only at frame boundaries.
-    __device__ __forceinline__ uint32_t* column() const { return G->state + i; }
-    __device__ __forceinline__ uint32_t& row(uint32_t w) const { return column()[(size_t)w * G->stride]; }
+    // The group through a pointer that the compiler cannot follow: the
+    // descriptor lies in constant memory, and it would load the fields that
+    // rare paths use ahead of the interpreter's loop and spill them.
+    __device__ __forceinline__ const FaGroup* grp() const
+    {
+        const FaGroup* g = G;
+#ifdef __CUDA_ARCH__
+        asm volatile("" : "+l"(g));
+#endif
+        return g;
+    }
+    __device__ __forceinline__ uint32_t* column() const { return grp()->state + i; }
+    __device__ __forceinline__ uint32_t& row(uint32_t w) const { return column()[(size_t)w * grp()->stride]; }
     __device__ __forceinline__ void fold_cycles()
     {
         uint32_t& lo = row(R_CYC_LO);
@@ -907,23 +1229,40 @@ struct Emu {
     __device__ __forceinline__ bool wsync() const { return (tw & TW_WSYNC) != 0; }
 
     // ------------------------------------------------------------ private bytes
-    __device__ __forceinline__ uint32_t poff(uint32_t o) const { return priv_off<BLOCK>(o); }
+    // Headless RAM: byte o of lane t at o * BLOCK + t, one multiply to reach;
+    // lanes at one offset share 8 words, at different offsets at most 4 of
+    // them meet in a bank.
+    __device__ __forceinline__ uint32_t poff(uint32_t o) const { return RENDER ? priv_off<BLOCK>(o) : o * BLOCK; }
     __device__ __forceinline__ uint32_t ldp(uint32_t o) const { return pv[poff(o)]; }
     __device__ __forceinline__ void stp(uint32_t o, uint32_t v) { pv[poff(o)] = (uint8_t)v; }
-    __device__ __forceinline__ uint32_t ldp16(uint32_t o) const { return *(const uint16_t*)(pv + poff(o)); }
-    __device__ __forceinline__ void stp16(uint32_t o, uint32_t v) { *(uint16_t*)(pv + poff(o)) = (uint16_t)v; }
 
     // ------------------------------------------------------------ flags
-    __device__ __forceinline__ void nz(uint32_t v) { p = (p & ~(F_N | F_Z)) | (v & F_N) | (v ? 0u : F_Z); }
-    __device__ __forceinline__ void setc(bool c) { p = (p & ~F_C) | (c ? F_C : 0u); }
+    __device__ __forceinline__ void set_nz(uint32_t v) { F = (F & 0xFFFF0000u) | v; }       // v: bytes 0 and 1
+    __device__ __forceinline__ void setc(uint32_t c) { F = (F & 0xFF00FFFFu) | (c << 16); }
+    __device__ __forceinline__ void setv(uint32_t v) { F = (F & 0x00FFFFFFu) | (v << 24); }
+    __device__ __forceinline__ uint32_t get_p() const
+    {
+        return p | (pd ? F_D : 0u) | ((F >> 16) & F_C) | ((F & 0xFFu) ? 0u : F_Z) | ((F >> 25) & F_V) | ((F | (F >> 8)) & F_N);
+    }
+    __device__ __forceinline__ void set_p(uint32_t v)
+    {
+        p = v & (F_I | F_B | F_U);
+        pd = (v & F_D) ? T_UV : 0u;
+        F = ((v & F_Z) ? 0u : 1u) | ((v & F_N) << 8) | ((v & F_C) << 16) | ((v & F_V) << 25);
+    }
+    // One more hotspot access this frame (a scheduling key only, saturating).
+    __device__ __forceinline__ void bump()
+    {
+        if ((kb & 0x01FF0000u) != 0x01FF0000u) kb += 0x10000u;
+    }
 
     // ------------------------------------------------------------ bank switching
     // A hotspot access selects its bank (src/atari.rs:460-492) and counts one
-    // more bank-switch point passed this frame in bank's upper bits.
+    // more bank-switch point passed this frame.
     __device__ __forceinline__ void bsw(uint32_t a13)
     {
-        uint32_t d = a13 - hot_lo;
-        if (d < nbanks) bank = (bank < (511u << 3) ? ((bank + 8u) & ~7u) : (bank & ~7u)) | d;
+        const uint32_t d = a13 - hot_lo;
+        if (d < nbanks) { bank = d << 12; bump(); }
     }
     // Sliced carts.  The ROM byte at a (A12 set): window (a >> 10) & 3 holds
     // slice `slices` byte k.
@@ -931,7 +1270,6 @@ struct Emu {
     {
         return (((slices >> ((a >> 7) & 0x18u)) & 0x1Fu) << 10) | (a & 0x3FFu);
     }
-    __device__ __forceinline__ void sbump() { bank = bank < (511u << 3) ? bank + 8u : bank; }
     // E0: any access to $1FE0-$1FF7 maps slice (a & 7) into window (a - $1FE0) >> 3.
     // DPC core: any access to $1FF8 / $1FF9 maps program bank 0 / 1 (slices 4b..4b+3).
     __device__ __forceinline__ void e0_hot(uint32_t a13)
@@ -939,16 +1277,22 @@ struct Emu {
         if constexpr (DPC) {
             if ((a13 | 1u) == 0x1FF9u) {
                 slices = (a13 & 1u) * 0x04040404u + 0x03020100u;
-                sbump();
+                bump();
             }
         } else {
             const uint32_t d = a13 - 0x1FE0u;
             if (d < 24u && fa_map_kind(hot_lo) == FA_MAP_E0) {
                 const uint32_t sh = (d >> 3) * 8u;
                 slices = (slices & ~(0xFFu << sh)) | ((a13 & 7u) << sh);
-                sbump();
+                bump();
             }
         }
+    }
+    // An access to ROM space: its hotspots.
+    __device__ __forceinline__ void hot(uint32_t a13)
+    {
+        if constexpr (!SLICED) bsw(a13);
+        else if constexpr (!FE) e0_hot(a13);
     }
     // The bank state (fa_state::mapper) to and from `slices`, for this core's
     // schemes only (fa_slices_from_mapper / fa_mapper_from_slices decode all
@@ -970,14 +1314,14 @@ struct Emu {
     {
         if (slices & 0x80u) {
             slices = ((v & 0x20u) ? 0u : 0x04040404u) + 0x03020100u;
-            sbump();
+            bump();
         }
         if (a13 == 0x01FEu) slices |= 0x80u;
     }
     // DPC core: reads of $1000-$103F and writes of $1040-$107F reach the registers.
     __device__ __forceinline__ uint32_t dpc(uint32_t a13, uint32_t v, uint32_t wr)
     {
-        return dpc_io(a13, v, wr, column(), G->stride, rom + 8192u, cyc_acc);
+        return dpc_io(a13, v, wr, column(), G->stride, rom + 8192u, cyc_acc + el);
     }
     // 3F: a write of v to $0000-$003F maps 2K bank v mod n at $1000-$17FF.
     __device__ __forceinline__ void f3_write(uint32_t a13, uint32_t v)
@@ -985,7 +1329,7 @@ struct Emu {
         if (a13 < 0x40u && fa_map_kind(hot_lo) == FA_MAP_3F) {
             const uint32_t b = v % (hot_lo & 0xFFu);
             slices = (slices & 0xFFFF0000u) | (2u * b) | ((2u * b + 1u) << 8);
-            sbump();
+            bump();
         }
     }
 
@@ -1009,6 +1353,36 @@ struct Emu {
         uint32_t c = (rem + 2u) / 3u;
         if (c) { clock = 228u; end_scanline(); }
         return c;
+    }
+    // Bring the beam, the timer's window and the cycle counter up to the d
+    // cycles counted so far (at an instruction boundary).  Only instructions
+    // that do not end the timer's window are counted, and only from a beam
+    // position and scanline in range (due() keeps dl at 0 otherwise), so the
+    // lines they complete fold together (tia_fold_io).
+    __device__ __forceinline__ void fold(uint32_t d)
+    {
+        const uint32_t clk = clock + 3u * d;
+        if (clk < 228u || d == 0u) {
+            clock = clk;
+        } else {
+            const uint4 r = tia_fold_io(clk, scanline | (pcnt << 16), tw);
+            clock = r.x; scanline = r.y & 0xFFFFu; pcnt = r.y >> 16; tw = r.z;
+        }
+        tlim -= d;
+        cyc_acc += d;
+    }
+    __device__ __forceinline__ void sync()
+    {
+        fold(el);
+        dl -= el;
+        el = 0;
+    }
+    // The cycles that may be counted before the frame loop must look: the
+    // timer's window, `lim` cycles to the frame limit, none while the beam is
+    // out of range (states only an upload makes; ticked one by one).
+    __device__ __forceinline__ uint32_t due(uint32_t lim) const
+    {
+        return (clock >= 228u || scanline >= 262u) ? 0u : tlim < lim ? tlim : lim;
     }
 
     // ------------------------------------------------------------ PIA timer (pia.rs:107-166)
@@ -1079,23 +1453,23 @@ struct Emu {
     // gives writes the Bus's timing (two TIA clocks, the write, one TIA clock
     // and the PIA clock); accesses to ROM and RAM do not depend on the beam
     // and are ticked with the rest of the instruction.
-    // Headless: ROM, RAM and hotspots are handled inline; TIA and PIA
-    // registers go through one out-of-line copy of their decoders (io_read /
-    // tia_write_io / pia_write_io), which keeps the interpreter's code small
-    // enough to stay resident in the instruction cache.
+    // Nothing here is a call in the headless console: a call costs some 50
+    // cycles and, worse, makes ptxas spill values of the interpreter's loop.
+    // The functions below serve exec(); run() has its own, narrower ones.
     __device__ __forceinline__ uint32_t io(uint32_t a, uint32_t j)   // TIA or PIA register read
     {
         if constexpr (RENDER) {
-            const uint32_t d = j - done;                              // cycles owed before this one
+            const uint32_t d = lag + j;                               // cycles owed before this one
             const RRead r = render_io_read(a, (int32_t)d > 0 ? d : 0u, rpack(), pins, pads, ports, pv, fbp);
             runpack(r.s);
-            done = j + 1u;
+            lag = 0u - (j + 1u);
             return r.v;
         } else {
             if ((a & 0x87u) == 0x84u) {                             // INTIM: settles and clears the flag
-                pia_intim();
+                intim();
                 return tp & 0xFFu;
             }
+            if ((a & 0x8Eu) == 0x08u) sync();                       // INPT0, INPT1: the paddle counter
             return io_read(a, pcnt, pins, pads, ports, su, (const uint8_t*)column(), G->stride * 4u);
         }
     }
@@ -1107,17 +1481,36 @@ struct Emu {
                 rsync(j);
                 r_write_cycle(a, v);
             } else {
-                const uint32_t d = j - done;
+                const uint32_t d = lag + j, t0 = tw;
                 runpack(render_write_cycle(a, v, (int32_t)d > 0 ? d : 0u, rpack(), pins, pv, fbp));
+                if (((tw ^ t0) & 0xFFu) || wsync()) done = 0;         // VSYNC changed, or a wait: the frame loop looks
             }
-            done = j + 1u;
-        } else if (a & 0x200u) {
-            const uint4 r = pia_store_io(a, v, ports, tp, su, tlim);
-            ports = r.x; tp = r.y; su = r.z; tlim = r.w;
+            lag = 0u - (j + 1u);
         } else {
-            uint2 r = tia_write_io(a, v, clock, tw, scanline | (pcnt << 16), (uint8_t*)column(), G->stride * 4u);
-            tw = r.x; scanline = r.y & 0xFFFFu; pcnt = r.y >> 16;
+            sync();
+            if (a & 0x200u) {
+                const uint4 r = pia_store_io(a, v, ports, tp, su, tlim);
+                ports = r.x; tp = r.y; su = r.z;
+                rewindow(r.w);
+            } else {
+                const uint2 r = tia_write_io(a, v, clock, tw, scanline | (pcnt << 16), (uint8_t*)column(), G->stride * 4u);
+                if ((r.x ^ tw) & (TW_WSYNC | 0xFFu)) dl = 0;          // a wait, or VSYNC changed: the frame loop looks
+                tw = r.x; scanline = r.y & 0xFFFFu; pcnt = r.y >> 16;
+            }
         }
+    }
+    // Headless, right after a sync: the timer has a new window.  A longer one
+    // leaves dl early, which only makes the frame loop look once too often.
+    __device__ __forceinline__ void rewindow(uint32_t w)
+    {
+        tlim = w;
+        dl = w < dl ? w : dl;
+    }
+    __device__ __forceinline__ void intim()
+    {
+        sync();
+        pia_intim();
+        rewindow(tlim);
     }
     __device__ __forceinline__ uint32_t read_low(uint32_t a, uint32_t j)   // a < 0x1000
     {
@@ -1144,7 +1537,7 @@ struct Emu {
                 return rom[srom(a)];
             } else {
                 bsw(a);
-                return rom[((bank & 7u) << 12) | (a & 0xFFFu)];
+                return rom[bank | (a & 0xFFFu)];
             }
         }
         if constexpr (FE) {
@@ -1192,7 +1585,7 @@ struct Emu {
             }
         } else if ((a & 0x287u) == 0x284u) {
             if constexpr (RENDER) (void)io(a, j);
-            else pia_intim();
+            else intim();
         }
     }
     __device__ __forceinline__ uint32_t zp_read(uint32_t z, uint32_t j)
@@ -1204,25 +1597,16 @@ struct Emu {
         }
         return (z & 0x80u) ? ldp(z & 0x7Fu) : io(z, j);
     }
-    __device__ __forceinline__ void push(uint32_t v, uint32_t j)
+    __device__ __forceinline__ void push(uint32_t sp, uint32_t v, uint32_t j)
     {
         if constexpr (FE) fe_note(0x100u | sp, v);
         if (sp & 0x80u) stp(sp & 0x7Fu, v); else io_write(0x100u | sp, v, j);
-        sp = (sp - 1u) & 0xFFu;
     }
-    __device__ __forceinline__ uint32_t pull(uint32_t j)
+    __device__ __forceinline__ uint32_t pull(uint32_t sp, uint32_t j)
     {
-        sp = (sp + 1u) & 0xFFu;
-        if constexpr (FE) {
-            const uint32_t v = (sp & 0x80u) ? ldp(sp & 0x7Fu)
-                                            : io_read(0x100u | sp, pcnt, pins, pads, ports, su, (const uint8_t*)column(),
-                                                      G->stride * 4u);
-            fe_note(0x100u | sp, v);
-            return v;
-        }
-        if (sp & 0x80u) return ldp(sp & 0x7Fu);
-        if constexpr (RENDER) return io(0x100u | sp, j);
-        else return io_read(0x100u | sp, pcnt, pins, pads, ports, su, (const uint8_t*)column(), G->stride * 4u);  // TIA
+        const uint32_t v = (sp & 0x80u) ? ldp(sp & 0x7Fu) : io(0x100u | sp, j);   // page 1 below $180 is TIA
+        if constexpr (FE) fe_note(0x100u | sp, v);
+        return v;
     }
     // Read-modify-write's two writes, on cycles j and j+1; a RAM target only
     // needs the second.
@@ -1236,369 +1620,521 @@ struct Emu {
         for (uint32_t m = 0; m < 2u; m++) write(ea, m ? newv : oldv, j + m);
     }
 
-    // ------------------------------------------------------------ ALU (cpu.rs:153-241)
-    __device__ __forceinline__ void adc(uint32_t v)
+    // ------------------------------------------------------------ instructions
+    // Instruction bytes at a0..a0+2 (13-bit) can be read together (FE: once the
+    // opcode is, which an access to $01FE before it lets select the bank): they lie in
+    // the current bank (SLICED: in one window) and clear of every hotspot
+    // (and, DPC, of its read registers at $1000-$103F), so reading them has no
+    // side effect.
+    __device__ __forceinline__ bool code_ok() const
     {
-        uint32_t c = p & F_C;
-        if (p & F_D) {
-            uint32_t lo = (a & 0xFu) + (v & 0xFu) + c;
-            if (lo > 9u) lo += 6u;
-            uint32_t hi = (a >> 4) + (v >> 4) + (lo > 0xFu ? 1u : 0u);
-            uint32_t bin = (a + v + c) & 0xFFu;
-            uint32_t res = ((hi << 4) | (lo & 0xFu)) & 0xFFu;
-            p &= ~(F_Z | F_N | F_V | F_C);
-            p |= bin ? 0u : F_Z;
-            p |= (hi & 8u) ? F_N : 0u;
-            p |= (~(a ^ v) & (a ^ res) & 0x80u) ? F_V : 0u;
-            if (hi > 9u) hi += 6u;
-            p |= hi > 0xFu ? F_C : 0u;
-            a = ((hi & 0xFu) << 4) | (lo & 0xFu);
-        } else {
-            uint32_t s = a + v + c;
-            uint32_t r = s & 0xFFu;
-            p = (p & ~(F_V | F_C)) | (s >> 8) | ((~(a ^ v) & (a ^ r) & 0x80u) ? F_V : 0u);
-            a = r;
-            nz(a);
-        }
+        const uint32_t a0 = pc & 0x1FFFu;
+        if constexpr (DPC) return a0 >= 0x1040u && (a0 & 0x3FFu) <= 0x3FDu && (a0 + 2u < 0x1FF8u || a0 > 0x1FF9u);
+        else if constexpr (FE) return a0 >= 0x1000u && (a0 & 0x3FFu) <= 0x3FDu;
+        else if constexpr (SLICED) return a0 >= 0x1000u && (a0 & 0x3FFu) <= 0x3FDu && (a0 + 2u < 0x1FE0u || a0 > 0x1FF7u);
+        else return (int32_t)(pc << 19) < (int32_t)((hot_lo - 2u) << 19);   // ROM addresses are negative, in order
     }
-    __device__ __forceinline__ void sbc(uint32_t v)
+    // ROM data at ea, below every hotspot: a load without a side effect
+    // (wr, T_WR or 0: and no write).
+    __device__ __forceinline__ bool data_ok(uint32_t ea, uint32_t wr = 0u) const
     {
-        uint32_t b = (p & F_C) ^ 1u;
-        int bin = (int)a - (int)v - (int)b;
-        uint32_t r = (uint32_t)bin & 0xFFu;
-        if (p & F_D) {
-            uint32_t lo = ((a & 0xFu) - (v & 0xFu) - b) & 0xFFu;
-            uint32_t lob = 0;
-            if (lo & 0x80u) { lo = (lo - 6u) & 0xFFu; lob = 1; }
-            uint32_t hi = ((a >> 4) - (v >> 4) - lob) & 0xFFu;
-            if (hi & 0x80u) hi = (hi - 6u) & 0xFFu;
-            p &= ~(F_Z | F_N | F_V | F_C);
-            p |= bin >= 0 ? F_C : 0u;
-            p |= r ? 0u : F_Z;
-            p |= r & F_N;
-            p |= ((a ^ v) & (a ^ r) & 0x80u) ? F_V : 0u;
-            a = ((hi & 0xFu) << 4) | (lo & 0xFu);
-        } else {
-            p = (p & ~(F_V | F_C)) | (bin >= 0 ? F_C : 0u) | (((a ^ v) & (a ^ r) & 0x80u) ? F_V : 0u);
-            a = r;
-            nz(a);
-        }
+        const int32_t s = (int32_t)((ea << 19) & ~(wr & T_WR));         // ROM addresses are negative, in order
+        if constexpr (DPC) return (uint32_t)s - (0x1040u << 19) < ((0x1FF8u - 0x1040u) << 19);
+        else if constexpr (FE) return s < 0;
+        else if constexpr (SLICED) return s < (int32_t)(0x1FE0u << 19);
+        else return s < (int32_t)(hot_lo << 19);                         // Fixed: hot_lo $2000, all of it
     }
-    __device__ __forceinline__ void cmp(uint32_t reg, uint32_t v)
-    {
-        setc(reg >= v);
-        nz((reg - v) & 0xFFu);
-    }
-    __device__ __forceinline__ void bit(uint32_t v)
-    {
-        p = (p & ~(F_Z | F_V | F_N)) | ((a & v) ? 0u : F_Z) | (v & (F_V | F_N));
-    }
-    // Shift/rotate/INC/DEC by the aaa field of a cc=10 opcode.
-    __device__ __forceinline__ uint32_t shift_op(uint32_t aaa, uint32_t v)
-    {
-        uint32_t r;
-        switch (aaa) {
-        case 0: setc(v & 0x80u); r = (v << 1) & 0xFFu; break;                       // ASL
-        case 1: r = ((v << 1) | (p & F_C)) & 0xFFu; setc(v & 0x80u); break;         // ROL
-        case 2: setc(v & 1u); r = v >> 1; break;                                    // LSR
-        case 3: r = (v >> 1) | ((p & F_C) << 7); setc(v & 1u); break;               // ROR
-        case 6: r = (v - 1u) & 0xFFu; break;                                        // DEC
-        default: r = (v + 1u) & 0xFFu; break;                                       // INC
-        }
-        nz(r);
-        return r;
-    }
+    __device__ __forceinline__ uint32_t rom_at(uint32_t a) const { return SLICED ? srom(a) : bank | (a & 0xFFFu); }
 
-    // ------------------------------------------------------------ instruction groups
-    // The opcode (at pc0) and the byte after it (b1: the operand, or the
-    // phantom read every 1-byte instruction makes at pc0+1) are read by
-    // step() for every legal opcode, in that order, as the reference does on
-    // cycles 1 and 2.  b2 is the byte at pc0+2 for the 3-byte forms, read on
-    // cycle 3 (JSR reads its high byte later and fetches it itself).
-
-    // cc = 01: ORA AND EOR ADC STA LDA CMP SBC x 8 addressing modes.
-    __device__ __forceinline__ uint32_t group1(uint32_t pc0, uint32_t aaa, uint32_t bbb, uint32_t b1, uint32_t b2)
+    // Executes instructions until one that may leave the lanes of a group at
+    // different pcs, one that reaches wait_key, or the end of the lane's
+    // frames.  After an instruction that the frame loop must look at (el
+    // reaches dl; RENDER: cyc_acc reaches done), look(cycles) does, and says
+    // whether the lane goes on: in the loop, since lanes are due at different
+    // times, and one that left would part from its group.  Returns 0 for an
+    // illegal opcode (pc is then past it and nothing else changed: the
+    // reference panics right after the opcode fetch, src/cpu.rs:1139-1141).
+    //
+    // What bounds it.  A lone warp on a scheduler: the dependent chain of
+    // three shared loads (23 cycles each: opcode, table, data) and some 25
+    // operations (5 each), and 11 cycles for every branch.  A full SM: the
+    // issue of its instructions, as long as the code in use stays within the
+    // 32 KB that the SM's instruction cache holds (2.5 times slower beyond).
+    // So operations, registers and flags are selected by the table's words
+    // instead of a switch (150 cycles for a lone warp), the loads are issued
+    // whatever the opcode needs (always from this lane's RAM or the ROM
+    // image), the frequent exceptions sit behind two tests, and the rest
+    // (exec) apart.  Measured on one B200, before (a switch decoder with the
+    // time kept per instruction) and now: 165 and 109 warp instructions, 1,290
+    // and 470 cycles per guest instruction of a lone warp; a frame of one
+    // plain cart 3.45 and 1.30 ms; the mixed batch of 135,500 consoles x 4
+    // frames 23.2 and 16.0 ms; a frame of 50,000 divergence carts 7.1 and 3.1 ms.
+    template <class LOOK>
+    __device__ __forceinline__ uint32_t run(uint32_t wait_key, LOOK look)
     {
-        const bool st = aaa == 4u;
-        uint32_t ea, cyc, v, base = 0;
-        bool indexed = false;                                       // (zp),Y, abs,Y, abs,X: a page may be crossed
-        switch (bbb) {
-        case 0: case 4: {
-            // (zp,X): the pointer at zp b1 + X, read on cycles 3-4; (zp),Y: at
-            // zp b1, on cycles 2-3.  One zero-page read loop for both.
-            const uint32_t z = bbb == 0u ? (b1 + x) & 0xFFu : b1, j0 = bbb == 0u ? 3u : 2u;
+        const sptr tab = to_sptr(op_table()), rs = to_sptr(rom), ps = to_sptr(pv);
+        uint32_t n;
+        const uint32_t end = instr + FA_BURST;
+#pragma unroll 1
+        do {
+            // Out of the window the loads stay inside the image: rom_at masks
+            // the offset, and the image is followed by other shared memory.
+            const bool ok = code_ok();
+            sptr q = rs + rom_at(pc);
+            const uint32_t op = lds8(q), slices0 = FE ? slices : 0u;
             if constexpr (FE) {
-                if (bbb == 0u) dummy(b1, 2);                        // the base, before X is added
+                if (ok & ((slices & 0x80u) != 0u)) { fe_note(pc & 0x1FFFu, op); q = rs + rom_at(pc); }
             }
-            uint32_t ptr = 0;
-#pragma unroll 1
-            for (uint32_t m = 0; m < 2u; m++) ptr |= zp_read((z + m) & 0xFFu, j0 + m) << (8u * m);
-            if (bbb == 0u) { ea = ptr; cyc = 6; }
-            else { base = ptr; ea = (ptr + y) & 0xFFFFu; cyc = 5; indexed = true; }
-            break;
-        }
-        case 1: ea = b1; cyc = 3; break;                            // zp
-        case 2: v = b1; cyc = 2; pc = (pc0 + 2u) & 0xFFFFu; goto operate;   // #imm ($89 is illegal)
-        case 3: ea = (b2 << 8) | b1; cyc = 4; break;                // abs
-        case 5:                                                     // zp,X
-            ea = (b1 + x) & 0xFFu; cyc = 4;
-            if constexpr (FE) dummy(b1, 2);                         // the base, before X is added
-            break;
-        default:                                                    // abs,Y / abs,X
-            base = (b2 << 8) | b1;
-            ea = (base + (bbb == 6u ? y : x)) & 0xFFFFu;
-            cyc = 4;
-            indexed = true;
-            break;
-        }
-        // The fix-up read at the unfixed address (every store, or a page crossed).
-        if (indexed && (st || ((base ^ ea) & 0xFF00u))) { dummy((base & 0xFF00u) | (ea & 0xFFu), cyc - 1u); cyc++; }
-        pc = (pc0 + ((bbb == 3u || bbb >= 6u) ? 3u : 2u)) & 0xFFFFu;
-        if (st) { write(ea, a, cyc - 1u); return cyc; }
-        v = read(ea, cyc - 1u);
-    operate:
-        switch (aaa) {
-        case 0: a |= v; nz(a); break;
-        case 1: a &= v; nz(a); break;
-        case 2: a ^= v; nz(a); break;
-        case 3: adc(v); break;
-        case 5: a = v; nz(a); break;
-        case 6: cmp(a, v); break;
-        default: sbc(v); break;
-        }
-        return cyc;
-    }
-
-    // cc = 10: ASL ROL LSR ROR STX LDX DEC INC, plus TXA TAX DEX NOP TXS TSX.
-    __device__ __forceinline__ uint32_t group2(uint32_t pc0, uint32_t aaa, uint32_t bbb, uint32_t b1, uint32_t b2)
-    {
-        uint32_t ea, cyc;
-        switch (bbb) {
-        case 0:                                                     // LDX #imm
-            x = b1; nz(x); pc = (pc0 + 2u) & 0xFFFFu; return 2;
-        case 2:                                                     // accumulator / implied
-            pc = (pc0 + 1u) & 0xFFFFu;
-            switch (aaa) {
-            case 4: a = x; nz(a); break;                            // TXA
-            case 5: x = a; nz(x); break;                            // TAX
-            case 6: x = (x - 1u) & 0xFFu; nz(x); break;             // DEX
-            case 7: break;                                          // NOP
-            default: a = shift_op(aaa, a); break;
-            }
-            return 2;
-        case 6:                                                     // TXS / TSX
-            pc = (pc0 + 1u) & 0xFFFFu;
-            if (aaa == 4u) sp = x; else { x = sp; nz(x); }
-            return 2;
-        case 1: ea = b1; cyc = 3; pc = (pc0 + 2u) & 0xFFFFu; break; // zp
-        case 3: ea = (b2 << 8) | b1; cyc = 4; pc = (pc0 + 3u) & 0xFFFFu; break;
-        case 5:                                                     // zp,X (zp,Y for STX/LDX)
-            ea = (b1 + ((aaa == 4u || aaa == 5u) ? y : x)) & 0xFFu; cyc = 4; pc = (pc0 + 2u) & 0xFFFFu;
-            if constexpr (FE) dummy(b1, 2);                         // the base, before the index is added
-            break;
-        default: {                                                  // abs,X (abs,Y for LDX)
-            pc = (pc0 + 3u) & 0xFFFFu;
-            const uint32_t base = (b2 << 8) | b1;
-            ea = (base + (aaa == 5u ? y : x)) & 0xFFFFu;
-            cyc = 4;
-            // LDX reads the unfixed address only when a page is crossed; the
-            // read-modify-write forms always do, and take 7 cycles.
-            if (aaa != 5u || ((base ^ ea) & 0xFF00u)) { dummy((base & 0xFF00u) | (ea & 0xFFu), 3); cyc = 5; }
-            break;
-        }
-        }
-        if (aaa == 4u) { write(ea, x, cyc - 1u); return cyc; }
-        if (aaa == 5u) { x = read(ea, cyc - 1u); nz(x); return cyc; }
-        const uint32_t v = read(ea, cyc - 1u);
-        rmw_store(ea, v, shift_op(aaa, v), cyc);
-        return cyc + 2u;
-    }
-
-    // cc = 00: control flow, stack, flags, BIT/STY/LDY/CPY/CPX.
-    // Bus-access sites are shared between the instructions of a group (one
-    // read and one write site for the memory forms, one push loop, one pull
-    // loop, one read loop for the new pc's bytes): every site is inlined code,
-    // and the interpreter's size decides how well it stays in the
-    // instruction cache.
-    __device__ __forceinline__ uint32_t group0(uint32_t pc0, uint32_t aaa, uint32_t bbb, uint32_t b1, uint32_t b2)
-    {
-        uint32_t ea, cyc, vb, vn, vs, vj, vv;
-        switch (bbb) {
-        case 4: {                                                   // branches
-            pc = (pc0 + 2u) & 0xFFFFu;
-            const uint32_t pos = (0x1067u >> (4u * (aaa >> 1))) & 0xFu;    // N V C Z
-            if (((p >> pos) & 1u) != (aaa & 1u)) return 2;
-            dummy(pc, 2);
-            const uint32_t npc = (pc + (uint32_t)(int32_t)(int8_t)(uint8_t)b1) & 0xFFFFu;
-            uint32_t bc = 3;
-            if ((pc ^ npc) & 0xFF00u) { dummy((pc & 0xFF00u) | (npc & 0xFFu), 3); bc = 4; }
-            pc = npc;
-            return bc;
-        }
-        case 6:                                                     // flags, TYA
-            pc = (pc0 + 1u) & 0xFFFFu;
-            switch (aaa) {
-            case 0: p &= ~F_C; break;
-            case 1: p |= F_C; break;
-            case 2: p &= ~F_I; break;
-            case 3: p |= F_I; break;
-            case 4: a = y; nz(a); break;
-            case 5: p &= ~F_V; break;
-            case 6: p &= ~F_D; break;
-            default: p |= F_D; break;
-            }
-            return 2;
-        case 2:                                                     // stack, DEY TAY INY INX
-            pc = (pc0 + 1u) & 0xFFFFu;
-            switch (aaa) {
-            case 4: y = (y - 1u) & 0xFFu; nz(y); return 2;          // DEY
-            case 5: y = a; nz(y); return 2;                         // TAY
-            case 6: y = (y + 1u) & 0xFFu; nz(y); return 2;          // INY
-            case 7: x = (x + 1u) & 0xFFu; nz(x); return 2;          // INX
-            default: break;
-            }
-            if (aaa & 1u) {                                         // PLP, PLA
-                if constexpr (FE) dummy(0x100u | sp, 2);            // the stack, before the pull
-                const uint32_t v = pull(3);
-                if (aaa == 1u) p = v & ~(F_B | F_U);
-                else { a = v; nz(a); }
-                return 4;
-            }
-            push(aaa == 0u ? (p | F_B | F_U) : a, 2);               // PHP, PHA
-            return 3;
-        case 0:
-            if (aaa < 2u) {                                         // BRK (b1 is the padding byte), JSR
-                const bool brk = aaa == 0u;
-                pc = (pc0 + 2u) & 0xFFFFu;
-                // BRK pushes pch, pcl, p on cycles 2-4; JSR pushes pch, pcl on
-                // cycles 3-4, before it reads the high byte.
-                const uint32_t n = brk ? 3u : 2u, j0 = brk ? 2u : 3u;
-                const uint32_t w = brk ? (pc << 8) | p | F_B | F_U : pc;
-                if constexpr (FE) {
-                    if (!brk) dummy(0x100u | sp, 2);                // JSR reads the stack before its pushes
+            const uint32_t b1 = lds8(q + 1), b2 = lds8(q + 2);
+            OpWord w = ldw(tab, op);
+            const uint32_t f = w.ix;
+            const uint32_t pc1 = pc + (w.rd >> 16);                   // past $FFFF: not ok, and exec() masks it
+            uint32_t base = __byte_perm(b1, b2, w.bs);
+            n = w.rs >> 16;
+            if (!ok | ((f & T_CTRL) != 0u)) {
+                if (!ok) goto exec_;
+                if (f & T_BR) {
+                    const bool tk = ((F & w.am) != 0u) != ((f & T_BI) != 0u);
+                    const uint32_t to = pc1 + (uint32_t)(int32_t)(int8_t)(uint8_t)b1;
+                    if (tk) n = 3u;
+                    if (tk & (((pc1 ^ to) & 0xFF00u) != 0u)) {        // the phantom read at the unfixed address
+                        if (!data_ok((pc1 & 0xFF00u) | (to & 0xFFu))) goto exec_;
+                        n = 4u;
+                    }
+                    pc = tk ? to : pc1;
+                    if (parted(tk) | ((int32_t)(instr - end) >= 0)) wait_key = 0u;   // leaves the loop
+                    goto done_;
                 }
-#pragma unroll 1
-                for (uint32_t k = 0; k < n; k++) push((w >> (8u * (n - 1u - k))) & 0xFFu, j0 + k);
-                if (brk) p |= F_I;
-                // BRK: the vector at $FFFE-$FFFF on cycles 5-6; JSR: the high
-                // byte at pc on cycle 5.
-                vb = brk ? 0xFFFEu : pc; vn = brk ? 2u : 1u; vs = brk ? 0u : 8u; vj = 5u; vv = brk ? 0u : b1;
-                cyc = brk ? 7u : 6u;
-                goto vector;
-            }
-            if (aaa < 4u) {                                         // RTI (p, pcl, pch), RTS (pcl, pch)
-                const bool rti = aaa == 2u;
-                const uint32_t n = rti ? 3u : 2u;
-                if constexpr (FE) dummy(0x100u | sp, 2);                // the stack, before the pulls
-                uint32_t w = 0;
-#pragma unroll 1
-                for (uint32_t k = 0; k < n; k++) w |= pull(3u + k) << (8u * k);
-                if (rti) {
-                    p = w & 0xFFu & ~(F_B | F_U);
-                    pc = w >> 8;
+                if (f & T_MEM) {
+                    // Through a zero-page pointer in RAM: its two bytes, then as
+                    // the absolute forms ((zp,X): no index left).
+                    const uint32_t z = (w.qs & (T_INDY << 16)) ? b1 : (b1 + ((R >> 8) & 0xFFu)) & 0xFFu;
+                    if (z - 0x80u >= 0x7Fu) goto exec_;
+                    base = lds8(ps + poff(z & 0x7Fu)) | (lds8(ps + poff((z + 1u) & 0x7Fu)) << 8);
                 } else {
-                    dummy(w, 5);
-                    pc = (w + 1u) & 0xFFFFu;
+                    const uint32_t o = (w.qs >> 16) & 63u;
+                    if (o == OP_JMP) { pc = b1 | (b2 << 8); goto done_; }
+                    uint32_t sp = R >> 24;
+                    if (o <= OP_JSR) {                                // PHP, PHA, JSR
+                        if (sp < 0x81u) goto exec_;
+                        const uint32_t u = o == OP_PHA ? R : o == OP_JSR ? (pc1 >> 8) : get_p() | F_B | F_U;
+                        if constexpr (FE) {
+                            if (o == OP_JSR) fe_note(0x100u | sp, lds8(ps + poff(sp & 0x7Fu)));   // JSR reads the stack first
+                            fe_note(0x100u | sp, u & 0xFFu);
+                        }
+                        sts8(ps + poff(sp & 0x7Fu), u);
+                        sp--;
+                        pc = pc1;
+                        if (o == OP_JSR) {
+                            sts8(ps + poff(sp & 0x7Fu), pc1);
+                            uint32_t hi = b2;
+                            if constexpr (FE) {
+                                fe_note(0x100u | sp, pc1 & 0xFFu);
+                                hi = lds8(rs + rom_at(pc1));          // its high byte comes last
+                                fe_note(pc1 & 0x1FFFu, hi);
+                            }
+                            sp--;
+                            pc = b1 | (hi << 8);
+                        }
+                    } else if (o >= OP_PLP && o <= OP_RTS) {
+                        if (sp - 0x7Fu >= (o == OP_RTS ? 0x7Fu : 0x80u) || (FE && sp < 0x80u)) goto exec_;
+                        const uint32_t u = lds8(ps + poff((sp + 1u) & 0x7Fu));
+                        if (o == OP_RTS) {
+                            const uint32_t ra = u | (lds8(ps + poff((sp + 2u) & 0x7Fu)) << 8);
+                            if (!data_ok(ra)) goto exec_;             // its phantom read
+                            if constexpr (FE) {
+                                fe_note(0x100u | sp, lds8(ps + poff(sp & 0x7Fu)));
+                                fe_note(0x101u + sp, u);
+                                fe_note(0x102u + sp, ra >> 8);
+                                fe_note(ra & 0x1FFFu, lds8(rs + rom_at(ra)));
+                            }
+                            sp++;
+                            pc = ra + 1u;
+                            wait_key = 0u;
+                        } else {
+                            if constexpr (FE) {
+                                fe_note(0x100u | sp, lds8(ps + poff(sp & 0x7Fu)));
+                                fe_note(0x101u + sp, u);
+                            }
+                            pc = pc1;
+                            if (o == OP_PLA) { R = (R & ~0xFFu) | u; set_nz(u); }
+                            else set_p(u & ~(F_B | F_U));
+                        }
+                        sp++;
+                    } else {
+                        goto exec_;
+                    }
+                    R = (R & 0xFFFFFFu) | (sp << 24);
+                    goto done_;
                 }
-                return 6;
             }
-            switch (aaa) {
-            case 5: y = b1; nz(y); break;                           // LDY #
-            case 6: cmp(y, b1); break;                              // CPY #
-            default: cmp(x, b1); break;                             // CPX #
-            }
-            pc = (pc0 + 2u) & 0xFFFFu;
-            return 2;
-        case 3:                                                     // absolute
-            pc = (pc0 + 3u) & 0xFFFFu;
-            if (aaa == 2u) { pc = (b2 << 8) | b1; return 3; }       // JMP
-            if (aaa == 3u) {                                        // JMP (ind), page-wrap bug
-                vb = (b2 << 8) | b1; vn = 2u; vs = 0u; vj = 3u; vv = 0u; cyc = 5u;
-                goto vector;
-            }
-            ea = (b2 << 8) | b1; cyc = 4;
-            break;
-        case 1:                                                     // zp: BIT STY LDY CPY CPX
-            pc = (pc0 + 2u) & 0xFFFFu;
-            ea = b1; cyc = 3;
-            break;
-        case 5:                                                     // zp,X: STY LDY
-            pc = (pc0 + 2u) & 0xFFFFu;
-            ea = (b1 + x) & 0xFFu; cyc = 4;
-            if constexpr (FE) dummy(b1, 2);                         // the base, before X is added
-            break;
-        default: {                                                  // abs,X: LDY
-            pc = (pc0 + 3u) & 0xFFFFu;
-            const uint32_t base = (b2 << 8) | b1;
-            ea = (base + x) & 0xFFFFu;
-            cyc = 4;
-            if ((base ^ ea) & 0xFF00u) { dummy((base & 0xFF00u) | (ea & 0xFFu), 3); cyc = 5; }
-            break;
-        }
-        }
-        return mem0(aaa, ea, cyc);
-    vector:                                                         // vn bytes from vb on, within its page
+            {
+                bool wr = (f & T_WR) != 0u;
+                const uint32_t ea = (base + __byte_perm(R, 0x80u, f)) & w.am;
+                const bool ram = ((ea & 0x1E80u) == 0x80u) & !(FE && (ea & 0x1FFFu) == 0x1FEu);
+                const sptr pr = ps + poff(ea & 0x7Fu), po = rs + rom_at(ea);
+                uint32_t ld = lds8(ram ? pr : po);
+                const bool plain = ram | data_ok(ea, f);
+                const bool far = ((base ^ ea) & 0xFF00u) != 0u;       // a page crossed
+                if (!plain | far | ((f & (pd | (T_ODD | T_FIX))) != 0u)) {
+                    const uint32_t o = (w.qs >> 16) & 63u;
+                    if (far | ((f & T_FIX) != 0u)) {
+                        // A fix-up read, at the base's page.  With the access
+                        // itself in plain ROM or RAM it is harmless unless that
+                        // page is $0F (the PIA's mirror), $1F (hotspots; an access
+                        // that wraps around) or, DPC, $10 (its registers).
+                        if (((base & 0xF00u) == 0xF00u) | (DPC && ((base & 0x1F00u) | (ea & 0xFFu)) - 0x1000u < 0x40u)) goto exec_;
+                        if (!plain & ((base & (FE ? 0x300u : 0x200u)) != 0u)) goto exec_;
+                        if (!(f & T_FIX)) n++;
+                    }
+                    if (!plain) {
+                        // ROM (a write, or a hotspot) or a register.
+                        const uint32_t a = ea & 0x1FFFu;
+                        const bool rmw = wr & (o < OP_STA);
+                        if constexpr (FE) {
+                            if (a == 0x1FEu) {                        // RAM, and the next access selects the bank
+                                if (rmw | ((f & (pd | T_ODD)) != 0u)) goto exec_;
+                                slices |= 0x80u;
+                                ld = lds8(pr);
+                                if (wr) sts8(pr, alu(w, ld, b1));
+                                commit(w, alu(w, ld, b1));
+                                pc = pc1;
+                                goto done_;
+                            }
+                        }
+                        if (!RENDER && (a & 0x1287u) == 0x284u && !intim_quick()) goto exec_;
+                        if (!wr | rmw) {
+                            const uint32_t j = n - (rmw ? 3u : 1u);
+                            if (a & 0x1000u) {
+                                hot(a);
+                                ld = (DPC && a < 0x1040u) ? dpc(a, 0u, 0u) : lds8(rs + rom_at(ea));
+                            } else {
+                                ld = bus_read(a, j);
+                            }
+                        }
+                        if (wr) {
+                            uint32_t r = alu(w, ld, b1);
+                            if (rmw) {
+                                if (f & T_ODD) r = shift(w, o, ld);
+                                F = __byte_perm(F, r, (f & T_ODD) ? 0x3574u : w.fs);
+                            }
 #pragma unroll 1
-        for (uint32_t m = 0; m < vn; m++) vv |= read((vb & 0xFF00u) | ((vb + m) & 0xFFu), vj + m) << (vs + 8u * m);
-        pc = vv;
-        return cyc;
-    }
-    __device__ __forceinline__ uint32_t mem0(uint32_t aaa, uint32_t ea, uint32_t cyc)
-    {
-        if (aaa == 4u) { write(ea, y, cyc - 1u); return cyc; }      // STY
-        const uint32_t v = read(ea, cyc - 1u);
-        switch (aaa) {
-        case 1: bit(v); break;
-        case 5: y = v; nz(y); break;
-        case 6: cmp(y, v); break;
-        default: cmp(x, v); break;
-        }
-        return cyc;
+                            for (uint32_t m = rmw ? 0u : 1u; m < 2u; m++) {
+                                const uint32_t u = (m ? r : ld) & 0xFFu;
+                                if (a & 0x1000u) {
+                                    hot(a);
+                                    if (DPC && a - 0x1040u < 0x40u) (void)dpc(a, u, 1u);
+                                } else {
+                                    bus_write(a, u, n - 2u + m);
+                                }
+                            }
+                            pc = pc1;
+                            goto done_;
+                        }
+                    }
+                    if (f & (pd | T_ODD)) {
+                        odd_op(w, o, ld, b1, pr, wr);
+                        wr = false;
+                        w.rd = w.fs = 0x3210u;                        // completed: nothing changes below
+                    }
+                }
+                const uint32_t r = alu(w, ld, b1);
+                if (wr) sts8(pr, r);
+                commit(w, r);
+                pc = pc1;
+                goto done_;
+            }
+        exec_:
+            if constexpr (FE) slices = slices0;                       // as before the opcode fetch
+            n = exec();
+            if (n == 0u) return 0u;
+            if (!ok | ((f & T_CTL) != 0u)) wait_key = 0u;
+        done_:
+            instr++;
+            if constexpr (RENDER) {
+                lag += n;
+                cyc_acc += n;
+            } else {
+                el += n;
+            }
+            if (RENDER ? cyc_acc >= done : el >= dl) {
+                if (!look(n)) break;
+            }
+        } while ((kb | pc) < wait_key);
+        return 1u;
     }
 
-    // One instruction; returns its cycle count, or 0 for an illegal opcode
-    // (pc is then past the opcode and nothing else changed: the reference
-    // panics right after the opcode fetch, src/cpu.rs:1139-1141).
-    __device__ __forceinline__ uint32_t step()
+    // The result of a table word's operation (byte 0), its carry (byte 1) and
+    // its V (bit 7 of byte 2): (s ^ v) + m (s & v) + q, with s ^ v left out for
+    // AND.  m = 2 adds (SBC and compares an inverted v), 1 ORs, 0 XORs; s = 0
+    // loads, v = 0 moves.
+    __device__ __forceinline__ uint32_t alu(const OpWord& w, uint32_t ld, uint32_t b1) const
     {
-        const uint32_t pc0 = pc;
-        const uint32_t a0 = pc0 & 0x1FFFu;
-        uint32_t op, b1, b2 = 0;
-        // Fast path: the three bytes at pc0 lie in the current bank (SLICED:
-        // in one window) and clear of every hotspot (and, DPC, of its read
-        // registers at $1000-$103F), so reading them has no side effect.
-        if (DPC      ? (a0 >= 0x1040u && (a0 & 0x3FFu) <= 0x3FDu && (a0 + 2u < 0x1FF8u || a0 > 0x1FF9u))
-            : FE     ? (a0 >= 0x1000u && (a0 & 0x3FFu) <= 0x3FDu && !(slices & 0x80u))     // not armed by $01FE
-            : SLICED ? (a0 >= 0x1000u && (a0 & 0x3FFu) <= 0x3FDu && (a0 + 2u < 0x1FE0u || a0 > 0x1FF7u))
-                     : (a0 >= 0x1000u && a0 + 2u < hot_lo)) {
-            const uint8_t* q = SLICED ? rom + srom(a0) : rom + ((bank & 7u) << 12) + (a0 & 0xFFFu);
-            op = q[0];
-            if (!((c_legal[op >> 5] >> (op & 31u)) & 1u)) { pc = (pc0 + 1u) & 0xFFFFu; return 0; }
+        const uint32_t s = __byte_perm(R, 0u, w.rs), v = __byte_perm(ld, b1, w.xs) ^ (w.am >> 16);
+        const uint32_t q = __byte_perm(F, 0xFF01u, w.qs);
+        const uint32_t r = ((s ^ v) & (uint32_t)((int32_t)w.qs >> 31)) + q + (s & v) * (w.bs >> 16);
+        return __byte_perm(r, (s ^ r) & (v ^ r), 0x3410u);
+    }
+    __device__ __forceinline__ void commit(const OpWord& w, uint32_t r)
+    {
+        R = __byte_perm(R, r, w.rd);
+        F = __byte_perm(F, r, w.fs);
+    }
+
+    // ASL, ROL, LSR, ROR of u: the result (byte 0) and its carry (byte 1).
+    __device__ __forceinline__ uint32_t shift(const OpWord& w, uint32_t o, uint32_t u) const
+    {
+        const uint32_t q = __byte_perm(F, 0xFF01u, w.qs);
+        return o <= OP_ROL ? (u << 1) | q : (u >> 1) | (q << 7) | ((u & 1u) << 8);
+    }
+
+    // Decimal ADC and SBC, and the T_ODD operations on A, RAM at pr (shifts
+    // that write) or the operand.
+    __device__ __forceinline__ void odd_op(const OpWord& w, uint32_t o, uint32_t ld, uint32_t b1, sptr pr, bool mem)
+    {
+        if (o == OP_ADC || o == OP_SBC) {
+            const uint32_t v = __byte_perm(ld, b1, w.xs), c = (F >> 16) & 1u;
+            const uint4 r = decimal_op(o == OP_SBC, R & 0xFFu, v, c);
+            R = (R & ~0xFFu) | r.x;
+            F = r.y | (r.z << 16) | ((r.w & 0x80u) << 24);
+        } else if (o >= OP_ASL && o <= OP_ROR) {
+            const uint32_t r = shift(w, o, mem ? ld : R & 0xFFu);
+            F = __byte_perm(F, r, 0x3574u);
+            if (mem) sts8(pr, r);
+            else R = __byte_perm(R, r, 0x3214u);
+        } else if (o == OP_BIT) {
+            set_nz((R & ld & 0xFFu) | ((ld & 0x80u) << 8));
+            setv(ld << 1);
+        } else if (o == OP_CLV) {
+            setv(0u);
+        } else if (o <= OP_SEI) {
+            p = o == OP_SEI ? p | F_I : p & ~F_I;
+        } else {
+            pd = o == OP_SED ? T_UV : 0u;
+        }
+    }
+
+    // Whether the lanes running this branch together part on it.
+    __device__ __forceinline__ static bool parted(bool tk)
+    {
+#ifdef __CUDA_ARCH__
+        const uint32_t am = __activemask(), tb = __ballot_sync(am, tk);
+        return (tb != 0u) & (tb != am);
+#else
+        (void)tk;
+        return true;
+#endif
+    }
+
+    // Headless: the timer is counting down with its underflow flag clear, so
+    // that an INTIM read changes nothing.
+    __device__ __forceinline__ bool intim_quick() const
+    {
+        return (su < 0x10000u) & (tlim != 0u) & ((tp & 0xFFFFu) != 0u);
+    }
+    // A read of a TIA or PIA register, or of a RAM mirror, at a < $1000
+    // outside $80-$FF and $180-$1FF (headless INTIM only if intim_quick).
+    __device__ __forceinline__ uint32_t bus_read(uint32_t a, uint32_t j)
+    {
+        if constexpr (RENDER) {
+            return read_low(a, j);
+        } else {
+            if (a & 0x80u) {
+                if (!(a & 0x200u)) return 0u;                        // never-written flat array
+                const uint32_t k = a & 7u;
+                // INTIM while the timer counts down: its value is that of the
+                // cycles left in the window (whole intervals and the prescaler).
+                if (k == 4u) return ((tlim - el - 1u) >> (__ffs(su) - 1)) + 1u;
+                if (k >= 4u) return k == 5u && su >= 0x10000u ? 0x80u : 0u;   // INSTAT
+                const uint32_t od = ports >> ((k & 2u) * 8u), ddr = (od >> 8) & 0xFFu;
+                const uint32_t in = pins >> ((k & 2u) * 4u);
+                return (k & 1u) ? ddr : ((in & ~ddr) | (od & ddr)) & 0xFFu;
+            }
+            const uint32_t r = a & 0x0Fu;
+            if (r < 8u) return (tw & TW_CX) ? ((const uint8_t*)column())[cold_off(PB_CX + r, grp()->stride * 4u)] : 0u;
+            if (r >= 12u) return ((pins >> (16u + (r & 1u))) & 1u) & (r < 14u ? 1u : 0u) ? 0x80u : 0u;
+            if (r >= 10u) return 0x80u;
+            sync();                                                  // INPT0, INPT1: the paddle counter
+            return pcnt >= ((pads >> (8u * (r & 1u))) & 0xFFu) ? 0x80u : 0u;
+        }
+    }
+    // A write at a < $1000 outside $80-$FF and $180-$1FF.
+    __device__ __forceinline__ void bus_write(uint32_t a, uint32_t v, uint32_t j)
+    {
+        if ((a & 0x280u) == 0x80u) { stp(a & 0x7Fu, v); return; }     // RAM mirrors
+        if constexpr (!RENDER) {
+            if (!(a & 0x200u)) {
+                const uint32_t r = a & 0x3Fu, e = tia_table()[r];
+                if (e) {                                              // a register that only keeps bits of v
+                    if constexpr (SLICED) f3_write(a, v);
+                    ((uint8_t*)column())[cold_off(e & 0xFFu, grp()->stride * 4u)] = (uint8_t)((v >> ((e >> 8) & 0xFFu)) & (e >> 16));
+                    return;
+                }
+            }
+        }
+        io_write(a, v, j);
+    }
+
+    // One instruction with every access on the bus, whatever it is.  What run()
+    // needs it for is rare: code near a hotspot or outside ROM, stacks and
+    // pointers that reach the TIA, phantom reads that may have side effects,
+    // BRK, RTI, JMP (ind), illegal opcodes.  It is inlined: as a call it cost
+    // the loop 30 registers' spills (a state in memory, and an ABI).
+    __device__ __forceinline__ uint32_t exec()
+    {
+        pc &= 0xFFFFu;
+        uint32_t b1, b2;
+        OpWord w;
+        if (code_ok() && !(FE && (slices & 0x80u))) {
+            const uint8_t* q = rom + rom_at(pc);
+            w = op_table()[q[0]];
             b1 = q[1];
             b2 = q[2];
         } else {
-            // The opcode, then its operand bytes, through one bus-read site.
-            uint32_t n = 2u, w = 0u;
-            op = 0u;
-#pragma unroll 1
-            for (uint32_t k = 0; k < n; k++) {
-                const uint32_t v = read((pc0 + k) & 0xFFFFu, k);
-                if (k == 0u) {
-                    op = v;
-                    if (!((c_legal[op >> 5] >> (op & 31u)) & 1u)) { pc = (pc0 + 1u) & 0xFFFFu; return 0; }
-                    const uint32_t bb = (op >> 2) & 7u;
-                    if (bb == 3u || bb == 7u || (bb == 6u && (op & 3u) == 1u)) n = 3u;
-                } else {
-                    w |= v << (8u * (k - 1u));
-                }
-            }
-            b1 = w & 0xFFu;
-            b2 = w >> 8;
+            fetch(b1, b2, w);
         }
-        const uint32_t aaa = op >> 5, bbb = (op >> 2) & 7u, cc = op & 3u;
-        if (cc == 1u) return group1(pc0, aaa, bbb, b1, b2);
-        if (cc == 2u) return group2(pc0, aaa, bbb, b1, b2);
-        return group0(pc0, aaa, bbb, b1, b2);
+        const uint32_t f = w.ix, o = (w.qs >> 16) & 63u;
+        if ((f & T_CTRL) && !(f & T_MEM)) return control(w, o, b1, b2);
+        pc = (pc + (w.rd >> 16)) & 0xFFFFu;
+        uint32_t n = w.rs >> 16, ld = 0;
+        if (f & T_MEM) {
+            uint32_t base = __byte_perm(b1, b2, w.bs);
+            if (w.qs & (T_IND << 16)) {
+                // (zp,X): the pointer at zp b1 + X, read on cycles 3-4; (zp),Y: at
+                // zp b1, on cycles 2-3.
+                const bool iy = (w.qs & (T_INDY << 16)) != 0u;
+                const uint32_t z = iy ? b1 : b1 + ((R >> 8) & 0xFFu), j0 = iy ? 2u : 3u;
+                if constexpr (FE) {
+                    if (!iy) dummy(b1, 2);                            // the base, before X is added
+                }
+                base = 0;
+#pragma unroll 1
+                for (uint32_t m = 0; m < 2u; m++) base |= zp_read((z + m) & 0xFFu, j0 + m) << (8u * m);
+            }
+            const uint32_t ea = (base + __byte_perm(R, 0x80u, f)) & w.am & 0xFFFFu;
+            const bool far = ((base ^ ea) & 0xFF00u) != 0u;
+            if (far && !(f & T_FIX)) n++;
+            if constexpr (FE) {
+                if (!(w.am & 0x100u) && (f & 7u) != 5u) dummy(b1, 2);   // zp,X / zp,Y: the base, before the index
+            }
+            const bool wr = (f & T_WR) != 0u, rmw = wr && o < OP_STA;
+            const uint32_t j = n - (rmw ? 3u : 1u);                   // the access's cycle, the fix-up read before it
+            if (far || (f & T_FIX)) dummy((base & 0xFF00u) | (ea & 0xFFu), j - 1u);
+            if (wr && !rmw) {
+                write(ea, __byte_perm(R, 0u, w.rs), j);
+                return n;
+            }
+            ld = read(ea, j);
+            if (rmw) {
+                uint32_t r;
+                r = (f & T_ODD) ? shift(w, o, ld) : alu(w, ld, b1);
+                F = __byte_perm(F, r, (f & T_ODD) ? 0x3574u : w.fs);
+                r &= 0xFFu;
+                rmw_store(ea, ld, r, n - 2u);
+                return n;
+            }
+        }
+        if (f & (pd | T_ODD)) odd_op(w, o, ld, b1, sptr(), false);
+        else commit(w, alu(w, ld, b1));
+        return n;
+    }
+
+    // The instruction's bytes one bus access at a time: code near a hotspot,
+    // outside ROM, or (FE) after an access to $01FE.
+    __device__ __forceinline__ void fetch(uint32_t& b1, uint32_t& b2, OpWord& w)
+    {
+        uint32_t n = 1u, u = 0u;
+#pragma unroll 1
+        for (uint32_t k = 0; k < n; k++) {
+            const uint32_t v = read((pc + k) & 0xFFFFu, k);
+            if (k == 0u) {
+                w = op_table()[v];
+                if (((w.qs >> 16) & 63u) != OP_ILL) n = (w.rd >> 16) == 3u ? 3u : 2u;
+            } else {
+                u |= v << (8u * (k - 1u));
+            }
+        }
+        b1 = u & 0xFFu;
+        b2 = u >> 8;
+        if (n != 3u) b2 |= 0x100u;                                    // JSR: not read yet
+    }
+
+    // Branches, stack and jumps.  Bus-access sites are shared (one push loop,
+    // one pull loop, one read loop for the new pc's bytes): every site is
+    // inlined code, and the code should fit the instruction cache.
+    __device__ __forceinline__ uint32_t control(const OpWord& w, uint32_t o, uint32_t b1, uint32_t b2)
+    {
+        uint32_t n = w.rs >> 16;
+        pc = (pc + (w.rd >> 16)) & 0xFFFFu;
+        if (w.ix & T_BR) {
+            if (((F & w.am) != 0u) == ((w.ix & T_BI) != 0u)) return n;   // not taken
+            const uint32_t to = (pc + (uint32_t)(int32_t)(int8_t)(uint8_t)b1) & 0xFFFFu;
+            n = 3;
+            const bool far = ((pc ^ to) & 0xFF00u) != 0u;
+            // The phantom read of the next opcode, and a far branch's at the
+            // unfixed address; in plain ROM neither has a side effect.
+            if (!code_ok()) dummy(pc, 2);
+            if (far) { dummy((pc & 0xFF00u) | (to & 0xFFu), 3); n = 4; }
+            pc = to;
+            return n;
+        }
+        if (o == OP_ILL) return 0u;
+        if (o == OP_JMP) { pc = (b1 | (b2 << 8)) & 0xFFFFu; return n; }
+        uint32_t vb, vn, vs = 0u, vj, vv = 0u;
+        if (o == OP_JMPI) {                                           // page-wrap bug
+            vb = (b1 | (b2 << 8)) & 0xFFFFu; vn = 2u; vj = 3u;
+        } else {
+            uint32_t sp = R >> 24;
+            if (o <= OP_BRK) {                                        // PHP, PHA, JSR, BRK
+                // BRK (b1 is the padding byte) pushes pch, pcl, p on cycles 2-4;
+                // JSR pushes pch, pcl on cycles 3-4, before it reads its high byte.
+                const uint32_t u = o == OP_PHA ? R : o == OP_JSR ? pc : (pc << 8) | get_p() | F_B | F_U;
+                const uint32_t m = o == OP_JSR ? 2u : o == OP_BRK ? 3u : 1u, j0 = o == OP_JSR ? 3u : 2u;
+                if constexpr (FE) {
+                    if (o == OP_JSR) dummy(0x100u | sp, 2);           // JSR reads the stack before its pushes
+                }
+#pragma unroll 1
+                for (uint32_t k = m; k-- > 0u;) {
+                    push(sp, (u >> (8u * k)) & 0xFFu, j0 + m - 1u - k);
+                    sp = (sp - 1u) & 0xFFu;
+                }
+                R = (R & 0xFFFFFFu) | (sp << 24);
+                if (o < OP_JSR) return n;
+                if (o == OP_JSR) {
+                    if (!FE && b2 < 0x100u) { pc = b1 | (b2 << 8); return n; }
+                    vb = pc; vn = 1u; vs = 8u; vv = b1;
+                } else {
+                    p |= F_I;
+                    vb = 0xFFFEu; vn = 2u;
+                }
+                vj = 5u;
+            } else {                                                  // PLP, PLA, RTS, RTI
+                const uint32_t m = o == OP_RTI ? 3u : o == OP_RTS ? 2u : 1u;
+                uint32_t u = 0;
+                if constexpr (FE) dummy(0x100u | sp, 2);              // the stack, before the pulls
+#pragma unroll 1
+                for (uint32_t k = 0; k < m; k++) {
+                    sp = (sp + 1u) & 0xFFu;
+                    u |= pull(sp, 3u + k) << (8u * k);
+                }
+                R = (R & 0xFFFFFFu) | (sp << 24);
+                if (o == OP_PLA) {
+                    R = (R & ~0xFFu) | u;
+                    set_nz(u);
+                } else if (o == OP_RTS) {
+                    dummy(u, 5);
+                    pc = (u + 1u) & 0xFFFFu;
+                } else {
+                    set_p(u & ~(F_B | F_U));
+                    if (o == OP_RTI) pc = (u >> 8) & 0xFFFFu;
+                }
+                return n;
+            }
+        }
+#pragma unroll 1
+        for (uint32_t m = 0; m < vn; m++) vv |= read((vb & 0xFF00u) | ((vb + m) & 0xFFu), vj + m) << (vs + 8u * m);
+        pc = vv;
+        return n;
     }
 
     // ------------------------------------------------------------ rendering console
@@ -1607,8 +2143,9 @@ struct Emu {
     // line (render_cycles / render_tia_ticks / render_io_read / render_write_cycle,
     // below), on the state they touch passed by value: one copy of the pixel
     // pipeline however many bus-access sites the interpreter has.
-    uint32_t done;            // cycle of the current instruction the TIA and PIA have reached (0 - lag at its start)
-    uint32_t lag;             // CPU cycles of earlier instructions not yet given to the TIA and PIA
+    uint32_t done;            // instruction cycles of the frame (cyc_acc) at which the frame loop must look
+    uint32_t lag;             // CPU cycles not yet given to the TIA and PIA; within an instruction, up to its start
+                             // (negative: they have reached cycle -lag of it)
     uint32_t vtop;            // visible_top | vblank_top << 16
     uint8_t* fbp;             // this instance's framebuffer, 160 x 192 palette indices
     uint32_t sc, zr;          // framebuffer sector in the sector buffer; rows written since the clear point | R_ZPEND
@@ -1634,8 +2171,8 @@ struct Emu {
     // given in one piece.
     __device__ __forceinline__ void rsync(uint32_t j)
     {
-        const uint32_t d = j - done;
-        if ((int32_t)d > 0) { runpack(render_cycles(rpack(), d, pins, pv, fbp)); done = j; }
+        const uint32_t d = lag + j;
+        if ((int32_t)d > 0) { runpack(render_cycles(rpack(), d, pins, pv, fbp)); lag = 0u - j; }
     }
     __device__ __forceinline__ void rcycles(uint32_t n) { runpack(render_cycles(rpack(), n, pins, pv, fbp)); }
     __device__ __forceinline__ void settle()
@@ -1706,9 +2243,9 @@ struct Emu {
     __device__ __forceinline__ void load_hot(const uint32_t* col, uint32_t stride)
     {
         uint32_t w;
-        w = col[R_AXYS * stride];  a = w & 0xFF; x = (w >> 8) & 0xFF; y = (w >> 16) & 0xFF; sp = w >> 24;
-        w = col[R_PC * stride];    pc = w & 0xFFFF; p = (w >> 16) & 0xFF; bank = w >> 24;
-        cyc_acc = 0;
+        R = col[R_AXYS * stride];
+        w = col[R_PC * stride];    pc = w & 0xFFFF; set_p((w >> 16) & 0xFF); bank = (w >> 24) << 12;
+        cyc_acc = 0; el = 0;
         const uint32_t p0 = col[R_PIA0 * stride];                  // pa_out pa_ddr pa_in pb_out
         const uint32_t p1 = col[R_PIA1 * stride];                  // pb_ddr pb_in uf pdump
         ports = (p0 & 0xFFFFu) | ((p0 >> 24) << 16) | ((p1 & 0xFFu) << 24);
@@ -1718,6 +2255,9 @@ struct Emu {
         w = col[R_TIA0 * stride];  clock = w & 0xFFFF; scanline = w >> 16;
         w = col[R_TIA1 * stride];                                   // wsync fcomp vsync vblank
         tw = ((w >> 16) & 0xFFFFu) | ((w & 1u) << 16) | (((w >> 8) & 1u) << 17) | (((p1 >> 24) & 1u) << 18);
+        if constexpr (!RENDER) {
+            if (col[(PB_CX / 4u) * stride] | col[(PB_CX / 4u + 1u) * stride]) tw |= TW_CX;
+        }
         if constexpr (SLICED) slices = slices_of(fa_tia1_mapper(w));
         w = col[R_TIA2 * stride];                                   // inpt4 inpt5 pad0 pad1
         pins = ((p0 >> 16) & 0xFFu) | (((p1 >> 8) & 0xFFu) << 8) | ((w & 1u) << 16) | (((w >> 8) & 1u) << 17);
@@ -1725,8 +2265,8 @@ struct Emu {
     }
     __device__ __forceinline__ void store_hot(uint32_t* col, uint32_t stride) const
     {
-        col[R_AXYS * stride] = a | (x << 8) | (y << 16) | (sp << 24);
-        col[R_PC * stride] = pc | (p << 16) | ((bank & 7u) << 24);
+        col[R_AXYS * stride] = R;
+        col[R_PC * stride] = pc | (get_p() << 16) | ((bank >> 12) << 24);
         col[R_PIA0 * stride] = (ports & 0xFFFFu) | ((pins & 0xFFu) << 16) | (((ports >> 16) & 0xFFu) << 24);
         col[R_PIA1 * stride] = (ports >> 24) | (((pins >> 8) & 0xFFu) << 8) | ((su >> 16) << 16) | (((tw >> 18) & 1u) << 24);
         const uint2 t = RENDER ? make_uint2(tp & 0xFFFFu, tp >> 16) : pia_now();
@@ -1741,15 +2281,24 @@ struct Emu {
     // RAM words from the HBM rows into shared memory and back.
     __device__ __forceinline__ void load_ram(const uint32_t* c, uint32_t stride)
     {
-        uint32_t* w = (uint32_t*)pv;
 #pragma unroll 4
-        for (uint32_t k = 0; k < FA_SMEM_WORDS; k++) w[k * BLOCK] = c[k * stride];
+        for (uint32_t k = 0; k < FA_SMEM_WORDS; k++) {
+            const uint32_t v = c[k * stride];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) pv[poff(4u * k + j)] = (uint8_t)(v >> (8u * j));
+        }
+    }
+    __device__ __forceinline__ uint32_t ram_word(uint32_t k) const
+    {
+        uint32_t v = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; j++) v |= (uint32_t)pv[poff(4u * k + j)] << (8u * j);
+        return v;
     }
     __device__ __forceinline__ void store_ram(uint32_t* c, uint32_t stride) const
     {
-        const uint32_t* w = (const uint32_t*)pv;
 #pragma unroll 4
-        for (uint32_t k = 0; k < FA_SMEM_WORDS; k++) c[k * stride] = w[k * BLOCK];
+        for (uint32_t k = 0; k < FA_SMEM_WORDS; k++) c[k * stride] = ram_word(k);
     }
 };
 

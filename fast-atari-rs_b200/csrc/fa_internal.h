@@ -16,8 +16,8 @@
 // Calls one fa_step_static may chain (one queue counter each in its fixed scratch).
 #define FA_STATIC_MAX_CALLS 1024
 // Dynamic shared memory a CTA may use (227 KiB opt-in limit minus the static
-// barrier word and headroom).
-#define FA_SMEM_PER_CTA_MAX (227 * 1024 - 1024)
+// opcode table, barrier word and headroom).
+#define FA_SMEM_PER_CTA_MAX (227 * 1024 - 8192 - 1024)
 
 // One cart's instance set in a launch.
 struct FaGroup {
@@ -65,6 +65,16 @@ struct FaLaunch {
     uint32_t trace_cap;          // units the trace holds
     const uint32_t* first_wave;  // warp-granular persistent form: the unit of each warp's first round
                                  // (index warp * grid + cta; ~0 for none), or null for warp * grid + cta
+};
+
+// The launchers of one build of the core (fa_core_kernels.cu, compiled once
+// per FA_MAPS_*): `warps` / `block` pick the kernel, sms <= 0 prepares only.
+template <int MAPS>
+struct FaCore {
+    static cudaError_t run_warps(int warps, const FaLaunch& L, bool persistent, int sms, cudaStream_t s);
+    static cudaError_t run_block(int block, const FaLaunch& L, bool persistent, int sms, cudaStream_t s);
+    static bool shape(int warps, const FaLaunch& L, bool persistent, int sms, uint32_t* grid, int* per_sm);
+    static int occupancy(int block, size_t smem);
 };
 
 // The launch shape fa_launch_run would use for L (warp-granular form only):

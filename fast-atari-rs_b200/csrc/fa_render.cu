@@ -68,6 +68,7 @@ __global__ void __maxnreg__(128) fa_render_run(const __grid_constant__ FaRenderL
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t rom_bytes = L.nbanks * 4096u;
     uint32_t* slab = (uint32_t*)(smem + rom_bytes) + warp * (FA_RSLAB_WORDS * 32u);
+    load_op_table();
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         FaGroup g;
@@ -112,6 +113,8 @@ __global__ void __maxnreg__(128) fa_render_run(const __grid_constant__ FaRenderL
     e.cyc_acc = 0;
     e.pc = 0;
     e.bank = 0;
+    e.kb = 0;
+    e.el = 0;
     e.slices = 0;
     e.scanline = 0;
     e.done = 0;

@@ -14,7 +14,8 @@ namespace fa {
 template <bool SLICED>
 struct RRunner {
     Emu<32, true, SLICED> e;
-    uint32_t f, phase, fcyc;
+    uint32_t f, phase;
+    uint32_t fcyc;           // WSYNC wait cycles of the frame (Emu::cyc_acc has its instruction cycles)
     bool active;
 
     // set_action, then run_frame, which does nothing for a halted console
@@ -26,80 +27,88 @@ struct RRunner {
         if (G->actions) e.apply_action(G->actions[(size_t)f * G->act_stride + e.i]);
         if (e.row(R_STATUS) & FA_STATUS_HALT_MASK) return false;
         e.tw &= ~TW_FCOMP;
-        e.bank &= 7u;
+        e.kb = (f < 0x7Fu ? f : 0x7Fu) << 25;
         fcyc = 0;
         phase = e.vsync_on() ? 0u : 1u;
+        e.done = due();
         return true;
     }
-    // One run_one_cycle: a WSYNC cycle (tick_components) or an instruction,
-    // then the frame-end checks of run_frame.
-    __device__ __forceinline__ bool one()
+    // The instruction cycles at which the frame loop must look: the VSYNC
+    // budget's or the frame cap's, less the frame's WSYNC waits.
+    __device__ __forceinline__ uint32_t due() const { return (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u - fcyc; }
+
+    // After an instruction (ran), the frame-end checks of run_frame, then any
+    // WSYNC wait it started, as a run_one_cycle of its own; until the frame
+    // loop has nothing to do at an instruction boundary.
+    __device__ __forceinline__ void attend(bool ran)
     {
-        uint32_t n;
-        if (e.wsync()) e.settle();                                   // the wait starts where the beam is
-        if (e.wsync()) {
+#pragma unroll 1
+        while (true) {
+            if (ran) {
+                const uint32_t fc = e.cyc_acc + fcyc;
+                if (phase == 0u) {
+                    if (fc > FA_VSYNC_BUDGET) {
+                        e.fold_cycles();
+                        e.set_status(FA_STATUS_VSYNC_BUDGET);
+                        active = false;
+                        return;
+                    }
+                    if (!e.vsync_on()) phase = 1u;
+                } else {
+                    const bool cap = fc > FA_FRAME_CYCLE_CAP;
+                    if (cap || e.vsync_on()) {
+                        if (cap) e.set_status(FA_STATUS_CYCLE_CAP);
+                        e.fb_observe();                              // before the next frame's action moves the pins
+                        e.fold_cycles();
+                        e.row(R_FRAME) += 1u;
+                        f++;
+                        if (f >= e.G->k || !begin_frame()) { active = false; return; }
+                    }
+                }
+            }
+            if (!e.wsync()) break;
+            e.settle();                                              // the wait starts where the beam is
+            if (!e.wsync()) break;
             // The cycles of a WSYNC wait up to the end of the line, cut where
             // a per-cycle frame check would first fire: nothing else changes
             // from one cycle of the wait to the next.
-            n = (228u - e.clock + 2u) / 3u;
-            uint32_t lim;
-            if (phase == 0u) lim = e.vsync_on() ? FA_VSYNC_BUDGET + 1u - fcyc : 1u;
-            else lim = FA_FRAME_CYCLE_CAP + 1u - fcyc;
+            uint32_t n = (228u - e.clock + 2u) / 3u, lim = 1u;
+            if (phase || e.vsync_on()) lim = due() - e.cyc_acc;
             n = n < lim ? n : lim;
             e.rcycles(n);
-        } else {
-            e.done = 0u - e.lag;
-            n = e.step();
-            if (n == 0) {
-                // The reference's opcode fetch was a bus access (one cycle of
-                // TIA and PIA) before it stopped (src/cpu.rs:1139-1141): the
-                // TIA and PIA are owed up to the end of that cycle.
-                e.lag = 1u - e.done;
-                e.fold_cycles();
-                e.set_status(FA_STATUS_ILLEGAL_OPCODE);
-                active = false;
-                return false;
-            }
-            e.lag = n - e.done;
-            e.instr++;
-            e.cyc_acc += n;
+            fcyc += n;
+            ran = true;
         }
-        fcyc += n;
-        if (phase == 0u) {
-            if (fcyc > FA_VSYNC_BUDGET) {
-                e.fold_cycles();
-                e.set_status(FA_STATUS_VSYNC_BUDGET);
-                active = false;
-                return false;
-            }
-            if (!e.vsync_on()) phase = 1u;
-        } else {
-            const bool cap = fcyc > FA_FRAME_CYCLE_CAP;
-            if (cap || e.vsync_on()) {
-                if (cap) e.set_status(FA_STATUS_CYCLE_CAP);
-                e.fb_observe();                                      // before the next frame's action moves the pins
-                e.fold_cycles();
-                e.row(R_FRAME) += 1u;
-                f++;
-                if (f >= e.G->k || !begin_frame()) { active = false; return false; }
-                return false;
-            }
-        }
-        return e.wsync();
+        e.done = due();
     }
+
     __device__ __forceinline__ uint32_t key(uint32_t sched) const
     {
-        const uint32_t fc = f < 0x7Fu ? f : 0x7Fu;
-        const uint32_t mid = sched == FA_SCHED_LINE ? (e.scanline < 0x1FFu ? e.scanline : 0x1FFu) : (e.bank >> 3);
-        return (fc << 25) | (mid << 16) | e.pc;
+        if (sched != FA_SCHED_LINE) return e.kb | e.pc;
+        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | e.pc;
     }
-    // A WSYNC wait is consumed without going back to the warp scheduler.
-    __device__ __forceinline__ void iterate()
+    __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | e.pc; }
+    // Instructions of this lane up to one that may leave the lanes of its
+    // group at different pcs, that reaches a waiting lane's key, or after
+    // which the frame loop must look (and the WSYNC waits it started).
+    __device__ __forceinline__ void burst(uint32_t wait_key)
     {
-#pragma unroll 1
-        while (one() && active) {
+        if (e.wsync()) {
+            attend(false);
+            if (!active) return;
+        }
+        if (!e.run(wait_key, [this](uint32_t) { attend(true); return active; })) {
+            // The reference's opcode fetch was a bus access (one cycle of TIA
+            // and PIA) before it stopped (src/cpu.rs:1139-1141): the TIA and
+            // PIA are owed up to the end of that cycle.
+            e.lag += 1u;
+            e.fold_cycles();
+            e.set_status(FA_STATUS_ILLEGAL_OPCODE);
+            active = false;
+            return;
         }
     }
+    __device__ __forceinline__ void iterate() { burst(0xFFFFFFFFu); }
 };
 
 }  // namespace fa

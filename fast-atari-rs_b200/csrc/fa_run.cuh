@@ -1,7 +1,7 @@
 // fa_run.cuh — device code shared by the library's kernels: bounded TMA bulk
 // staging on an mbarrier, and the per-unit runner (frame loop, warp
 // scheduling policies, one unit of instances from HBM rows to HBM rows).
-// Included by fa_kernels.cu (pool/handle kernels) and fa_serve_kernel.cu
+// Included by fa_core_kernels.cu (pool/handle kernels) and fa_serve_kernel.cu
 // (serving kernel, compiled with L1-bypassing global loads).
 #pragma once
 #include <cuda_runtime.h>
@@ -103,7 +103,8 @@ static __device__ bool stage_rom(uint8_t* dst, const uint8_t* src, uint32_t byte
 template <int BLOCK, bool SLICED = false, bool DPC = false, bool FE = false>
 struct Runner {
     Emu<BLOCK, false, SLICED, DPC, FE> e;
-    uint32_t f, phase, fcyc;
+    uint32_t f, phase;
+    uint32_t fcyc;           // WSYNC wait cycles of the frame (Emu::cyc_acc has its instruction cycles)
     bool active;
 
     // Start frame f in the order of one frame of a batched step: the
@@ -112,7 +113,7 @@ struct Runner {
     // instance is halted: its inputs still take the frame's action.
     __device__ __forceinline__ bool begin_frame()
     {
-        const FaGroup* G = e.G;
+        const FaGroup* G = e.grp();
         if (G->episode_frames && G->snapshot && e.row(R_FRAME) >= G->episode_frames) {
             e.load_ram(G->snapshot, 1);
             // The DPC rows only for the DPC core: they stay 0 for every other
@@ -126,48 +127,81 @@ struct Runner {
         if (e.row(R_STATUS) & FA_STATUS_HALT_MASK) return false;
         e.tw &= ~TW_FCOMP;
         fcyc = 0;
-        e.bank &= 7u;
+        e.kb = (f < 0x7Fu ? f : 0x7Fu) << 25;
         phase = e.vsync_on() ? 0u : 1u;
+        e.dl = e.wsync() ? 0u : due();
         return true;
     }
 
-    // One HeadlessAtari::run_one_cycle (src/atari.rs:601-614) plus the frame
-    // loop checks of run_frame (src/atari.rs:584-598).  Returns true when the
-    // lane should run again immediately (a WSYNC skip is pending).
-    __device__ __forceinline__ bool one()
+    // Cycles until the frame loop must look again (Emu::dl): the timer's
+    // window, the VSYNC budget or the frame's cycle cap.  The frame's elapsed
+    // cycles are its instruction cycles and its WSYNC waits (fcyc).
+    __device__ __forceinline__ uint32_t due() const
     {
-        uint32_t n;
-        if (e.wsync()) {
-            n = e.tia_skip();
-        } else {
-            n = e.step();
-            if (n == 0) { e.fold_cycles(); e.set_status(FA_STATUS_ILLEGAL_OPCODE); active = false; return false; }
-            e.instr++;
-            e.cyc_acc += n;
+        return e.due((phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u - (e.cyc_acc + fcyc));
+    }
+
+    // One HeadlessAtari::run_one_cycle (src/atari.rs:601-614) after another
+    // until the frame loop has nothing to do at an instruction boundary: the
+    // ticks of the instruction of n cycles just executed (n = 0: none), the
+    // checks of run_frame (src/atari.rs:584-598), then any WSYNC wait it
+    // started, as a run_one_cycle of its own.
+    __device__ __forceinline__ void attend(uint32_t n)
+    {
+        e.fold(e.el - n);
+        e.el = 0;
+        if (n) {
             e.tia_tick(n);
+            e.cyc_acc += n;
         }
-        e.pia_count(n);
-        fcyc += n;
-        if (phase == 0u) {
-            if (fcyc > FA_VSYNC_BUDGET) {
-                e.fold_cycles();
-                e.set_status(FA_STATUS_VSYNC_BUDGET);
-                active = false;
-                return false;
+#pragma unroll 1
+        while (true) {
+            if (n) {
+                e.pia_count(n);
+                const uint32_t fc = e.cyc_acc + fcyc;
+                if (phase == 0u) {
+                    if (fc > FA_VSYNC_BUDGET) {
+                        e.fold_cycles();
+                        e.set_status(FA_STATUS_VSYNC_BUDGET);
+                        active = false;
+                        return;
+                    }
+                    if (!e.vsync_on()) phase = 1u;
+                } else {
+                    const bool cap = fc > FA_FRAME_CYCLE_CAP;
+                    if (cap || e.vsync_on()) {
+                        if (cap) e.set_status(FA_STATUS_CYCLE_CAP);
+                        e.fold_cycles();
+                        e.row(R_FRAME) += 1u;
+                        f++;
+                        if (f >= e.grp()->k || !begin_frame()) { active = false; return; }
+                    }
+                }
             }
-            if (!e.vsync_on()) phase = 1u;
-        } else {
-            const bool cap = fcyc > FA_FRAME_CYCLE_CAP;
-            if (cap || e.vsync_on()) {
-                if (cap) e.set_status(FA_STATUS_CYCLE_CAP);
-                e.fold_cycles();
-                e.row(R_FRAME) += 1u;
-                f++;
-                if (f >= e.G->k || !begin_frame()) { active = false; return false; }
-                return false;
-            }
+            if (!e.wsync()) break;
+            n = e.tia_skip();
+            if (n == 0u) break;
+            fcyc += n;
         }
-        return e.wsync();
+        e.dl = due();
+    }
+
+    // Instructions of this lane up to one that may leave the lanes of its
+    // group at different pcs, that reaches a waiting lane's key, or after
+    // which the frame loop must look (and the WSYNC waits it started).
+    __device__ __forceinline__ void burst(uint32_t wait_key)
+    {
+        if (e.wsync()) {                                              // a wait pending at the call's or frame's start
+            attend(0u);
+            if (!active) return;
+        }
+        if (!e.run(wait_key, [this](uint32_t n) { attend(n); return active; })) {
+            e.sync();
+            e.fold_cycles();
+            e.set_status(FA_STATUS_ILLEGAL_OPCODE);
+            active = false;
+            return;
+        }
     }
 
     // Scheduling key, a measure of how far the lane has progressed: frame,
@@ -175,31 +209,20 @@ struct Runner {
     // address in two banks is two program points, and a lane that has
     // switched banks once more is ahead whatever its pc) or the scanline
     // (FA_SCHED_LINE), then pc.
-    __device__ __forceinline__ uint32_t key(uint32_t sched) const
+    __device__ __forceinline__ uint32_t key(uint32_t sched)
     {
-        const uint32_t fc = f < 0x7Fu ? f : 0x7Fu;
-        const uint32_t mid = sched == FA_SCHED_LINE ? (e.scanline < 0x1FFu ? e.scanline : 0x1FFu) : (e.bank >> 3);
-        return (fc << 25) | (mid << 16) | e.pc;
+        if (sched != FA_SCHED_LINE) return e.kb | e.pc;
+        e.sync();
+        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | e.pc;
     }
-
-    // Up to three run_one_cycle calls per scheduler step (an instruction, a
-    // WSYNC skip it starts, one more); on the mixed batch this measured 4 %
-    // faster than two (19.4 against 18.6 M frames/s on one B200), with the
-    // same results, since the policy only changes when lanes are polled.
-    __device__ __forceinline__ void iterate()
-    {
-#pragma unroll 1
-        for (int rep = 0; rep < 3; rep++)
-            if (!one() || !active) break;
-    }
+    // Where the lane is: pc, bank and bank-switch count.
+    __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | e.pc; }
+    __device__ __forceinline__ void iterate() { burst(0xFFFFFFFFu); }
 };
 
 // Runs every lane of the warp to the end of its frames.  The policy only
 // decides which lanes execute in each round; all lanes share one call site of
 // the emulator so its code is instantiated once.
-// Instructions a converged group may run per scheduling round.
-constexpr uint32_t FA_STEPS_PER_ROUND = 32;
-
 template <class RUNNER>
 __device__ __forceinline__ uint32_t run_lanes(RUNNER& r, uint32_t sched)
 {
@@ -209,9 +232,9 @@ __device__ __forceinline__ uint32_t run_lanes(RUNNER& r, uint32_t sched)
     uint32_t rem = 0, grp = 0, rounds = 0;
     while (true) {
         const bool act = r.active;
-        const uint32_t pcb = (r.e.bank << 16) | r.e.pc;
+        const uint32_t pcb = r.place();
         bool go;
-        uint32_t gm = FULL, lead = 0, wait_key = 0;
+        uint32_t gm = FULL, lead = 0, wait_key = 0xFFFFFFFFu;
         if (sched == FA_SCHED_MATCH) {
             // __match_any_sync groups lanes by (bank, pc); each group runs its
             // instruction together, every group once per round.
@@ -241,31 +264,32 @@ __device__ __forceinline__ uint32_t run_lanes(RUNNER& r, uint32_t sched)
             // running only while every member's key stays below it (so it
             // stops where a waiting lane could join); it may stop earlier than
             // needed, never later, so the order of execution is the one
-            // one-instruction rounds would follow.
+            // one-instruction rounds would follow.  The line policy's keys
+            // move with the beam: with lanes waiting, one instruction a check.
             wait_key = __reduce_min_sync(FULL, go ? 0xFFFFFFFFu : key);
         } else {
             if (!__any_sync(FULL, act)) break;
             go = act;
         }
         // One call site of the emulator for every policy.  A converged group
-        // keeps running (up to FA_STEPS_PER_ROUND instructions) while its
-        // lanes stay at one pc: one shuffle and one vote per instruction
-        // instead of a full scheduling round.  With no lane waiting
-        // (wait_key all ones, the common fully converged warp) the keys need
-        // not be compared.
-        uint32_t steps = 0;
+        // keeps running while its lanes stay at one pc: one shuffle and one
+        // vote after each instruction that may part them, instead of a full
+        // scheduling round.  The other policies part the lanes' rounds at the
+        // same instructions.
+        uint32_t ran = 0;
         if (go) {
+            const uint32_t i0 = r.e.instr;
+            const uint32_t stop = sched == FA_SCHED_LINE && wait_key != 0xFFFFFFFFu ? 0u : wait_key;
             while (true) {
-                r.iterate();
-                if (!converge || ++steps >= FA_STEPS_PER_ROUND) break;
-                const uint32_t mp = (r.e.bank << 16) | r.e.pc;
+                r.burst(stop);
+                if (!converge) break;
+                const uint32_t mp = r.place();
                 const uint32_t lp = __shfl_sync(gm, mp, lead);
-                const bool cont = wait_key == 0xFFFFFFFFu ? (r.active && mp == lp)
-                                                          : (r.active && mp == lp && r.key(sched) < wait_key);
-                if (!__all_sync(gm, cont)) break;
+                if (!__all_sync(gm, r.active && mp == lp && (wait_key == 0xFFFFFFFFu || r.key(sched) < wait_key))) break;
             }
+            ran = r.e.instr - i0;
         }
-        rounds += converge ? __shfl_sync(FULL, steps, lead) : 1u;
+        rounds += converge ? __shfl_sync(FULL, ran, lead) : ~__reduce_min_sync(FULL, ~ran);   // the most of any lane
     }
     return rounds;
 }
@@ -282,7 +306,7 @@ __device__ __forceinline__ void run_unit_as(const FaGroup& G, uint32_t first, ui
     r.phase = 0;
     r.fcyc = 0;
     r.active = false;
-    r.e.pv = (uint8_t*)(priv + t);
+    r.e.pv = (uint8_t*)priv + t;
     r.e.G = &G;
     r.e.i = first + t;
     r.e.rom = rom_s;
@@ -292,6 +316,9 @@ __device__ __forceinline__ void run_unit_as(const FaGroup& G, uint32_t first, ui
     r.e.cyc_acc = 0;
     r.e.pc = 0;
     r.e.bank = 0;
+    r.e.kb = 0;
+    r.e.el = 0;
+    r.e.dl = 0;
     r.e.slices = 0;
     r.e.scanline = 0;
     const bool valid = t < count;
@@ -311,12 +338,11 @@ __device__ __forceinline__ void run_unit_as(const FaGroup& G, uint32_t first, ui
         r.e.store_ram(col, G.stride);
         r.e.store_hot(col, G.stride);
         if (G.obs) {
-            const uint32_t* w = priv + t;
             uint4* o = (uint4*)(G.obs + (size_t)r.e.i * 128u);
-#pragma unroll
+#pragma unroll 2
             for (uint32_t q = 0; q < 8u; q++)
-                o[q] = make_uint4(w[(4u * q) * BLOCK], w[(4u * q + 1u) * BLOCK], w[(4u * q + 2u) * BLOCK],
-                                  w[(4u * q + 3u) * BLOCK]);
+                o[q] = make_uint4(r.e.ram_word(4u * q), r.e.ram_word(4u * q + 1u), r.e.ram_word(4u * q + 2u),
+                                  r.e.ram_word(4u * q + 3u));
         }
     }
     if (instr_out) {

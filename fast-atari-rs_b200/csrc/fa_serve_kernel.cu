@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) fa_serve(const __grid_
     uint32_t* priv = (uint32_t*)(smem + rom_bytes) + warp * (FA_SMEM_WORDS * 32u);
     const uint32_t u = blockIdx.x * WARPS + warp;
     const bool have = u < L.nunits;
+    load_op_table();
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     if (have && lane == 0) {
         const FaServeUnit U = L.unit[u];
