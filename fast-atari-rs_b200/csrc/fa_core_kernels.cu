@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(WARPS * 32) fa_run_warps(const __grid_constant
     __shared__ __align__(8) uint64_t bar;
     const uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    uint32_t* priv = (uint32_t*)(smem + L.romlib_bytes) + warp * (FA_SMEM_WORDS * 32u);
+    uint32_t* priv = (uint32_t*)(smem + L.romlib_bytes) + warp * (fa_slab_words(MAPS) * 32u);
 
     load_op_table();
     if (threadIdx.x == 0) mbar_init(&bar, 1);
@@ -136,7 +136,7 @@ int per_sm_for(size_t smem)
     if (it != g_per_sm.end()) return it->second;
     const auto max_key = std::make_pair(dev, std::make_pair(BLOCK * 4 + SL, (size_t)0));
     if (g_per_sm.find(max_key) == g_per_sm.end()) {
-        const int max_smem = 32768 + FA_SMEM_WORDS * BLOCK * 4;
+        const int max_smem = 32768 + fa_slab_words(SL) * BLOCK * 4;
         if (cudaFuncSetAttribute(fa::fa_run<BLOCK, SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) !=
             cudaSuccess)
             return -1;
@@ -153,7 +153,7 @@ int per_sm_for(size_t smem)
 template <int BLOCK, int SL>
 static cudaError_t launch_block(const FaLaunch& L, bool persistent, int sms, cudaStream_t s)
 {
-    const size_t smem = (size_t)L.rom_bytes_max + (size_t)FA_SMEM_WORDS * BLOCK * 4u;
+    const size_t smem = (size_t)L.rom_bytes_max + (size_t)fa_slab_words(SL) * BLOCK * 4u;
     const int per_sm = per_sm_for<BLOCK, SL>(smem);
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     if (sms <= 0) return cudaSuccess;                                  // prepare only
@@ -197,7 +197,7 @@ int warps_per_sm_for(size_t smem)
 template <int WARPS, int SL>
 cudaError_t launch_warps(const FaLaunch& L, bool persistent, int sms, cudaStream_t s)
 {
-    const size_t smem = (size_t)L.romlib_bytes + (size_t)WARPS * FA_SMEM_WORDS * 32u * 4u;
+    const size_t smem = (size_t)L.romlib_bytes + (size_t)WARPS * fa_slab_words(SL) * 32u * 4u;
     const int per_sm = warps_per_sm_for<WARPS, SL>(smem);
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     if (sms <= 0) return cudaSuccess;                                  // prepare only
@@ -218,7 +218,7 @@ cudaError_t launch_warps(const FaLaunch& L, bool persistent, int sms, cudaStream
 template <int WARPS, int SL>
 void warps_shape(const FaLaunch& L, bool persistent, int sms, uint32_t* grid, int* per_sm)
 {
-    const size_t smem = (size_t)L.romlib_bytes + (size_t)WARPS * FA_SMEM_WORDS * 32u * 4u;
+    const size_t smem = (size_t)L.romlib_bytes + (size_t)WARPS * fa_slab_words(SL) * 32u * 4u;
     *per_sm = warps_per_sm_for<WARPS, SL>(smem);
     uint32_t g = (L.nunits + WARPS - 1) / WARPS;
     if (persistent) {

@@ -57,8 +57,8 @@ struct alignas(16) OpWord {
     uint32_t rs;   // over (registers, 0): the register operand; high half: cycles without the page-crossing and branch penalties
     uint32_t rd;   // over (registers, result): the new registers; high half: bytes
     uint32_t bs;   // over (operand bytes): the base address; high half: m of Emu::alu
-    uint32_t qs;   // over (flags, 1, $FF, 0): what is added; high half: OP_* | T_IND, T_INDY, T_K
-    uint32_t fs;   // over (flags, result and its flags): the new flags
+    uint32_t qs;   // over (flags, 1, $FF, 0): what is added; high half: OP_* | T_IND, T_INDY
+    uint32_t fs;   // over (flags, result and its flags): the new flags; high half: k of Emu::alu
     uint32_t am;   // address mask, $FF (wraps in zero page) or $FFFF; high half: what the operand is XORed with.  Branches: the flag tested
     uint32_t xs;   // over (memory operand, first operand byte): the operand
 };
@@ -73,8 +73,7 @@ enum : uint32_t {                                                     // in ix
     T_CTL = 1u << 28,     // may leave lanes of a converged group at different pcs
     T_ODD = 1u << 29,     // shifts, BIT, operations on I, D and V
 };
-// With the operation: through a zero-page pointer, (zp),Y; the XOR term of Emu::alu kept (all but AND).
-enum : uint32_t { T_IND = 0x40u, T_INDY = 0x80u, T_K = 0x8000u };
+enum : uint32_t { T_IND = 0x40u, T_INDY = 0x80u };                    // with the operation: through a zero-page pointer, (zp),Y
 enum : uint32_t {
     // on a value read (memory or immediate)
     OP_ORA, OP_AND, OP_EOR, OP_ADC, OP_LDA, OP_CMP, OP_SBC, OP_LDX, OP_LDY, OP_CPX, OP_CPY, OP_BIT,
@@ -104,7 +103,7 @@ constexpr OpTable make_op_table()
                           0xFFu, 0x1111u };
     auto set = [&](uint32_t op, uint32_t o, uint32_t mode, uint32_t idx, uint32_t flags, uint32_t ind, uint32_t len,
                    uint32_t cyc) {
-        uint32_t src = N, dst = N, q = Q0, b = 0, m = 1, f = 0, kx = T_K;
+        uint32_t src = N, dst = N, q = Q0, b = 0, m = 1, f = 0, kx = 1;
         bool nz = true, c = false, v = false, use = true;            // use: the operand enters the result
         switch (o) {
         case OP_ORA: src = dst = A; break;
@@ -149,7 +148,7 @@ constexpr OpTable make_op_table()
         const uint32_t d = dst == N ? 0x3210u : (0x3210u & ~(0xFu << (4u * dst))) | (4u << (4u * dst));
         const uint32_t fl = (nz ? 0x74u : 0x10u) | (c ? 0x500u : 0x200u) | (v ? 0x6000u : 0x3000u);
         t.e[op] = OpWord{ 0x5550u | i | f | flags, 0x4440u | src | (cyc << 16), d | (len << 16),
-                          (mode == ZP ? 0x1110u : mode == AB ? 0x1140u : 0x1111u) | (m << 16), 0x6660u | q | ((o | ind | kx) << 16), fl,
+                          (mode == ZP ? 0x1110u : mode == AB ? 0x1140u : 0x1111u) | (m << 16), 0x6660u | q | ((o | ind) << 16), fl | (kx << 16),
                           (mode == AB ? 0xFFFFu : 0xFFu) | (b << 16),
                           !use ? 0x1111u : mem ? 0x1110u : mode == IM ? 0x1114u : 0x1111u };
     };
@@ -236,6 +235,18 @@ constexpr TiaTable make_tia_table()
     return t;
 }
 
+// v in a register of its own: not loaded or computed again from the launch's
+// constants wherever it is used, which ptxas otherwise prefers to keeping it
+// (4 constant loads and 12 more instructions per guest instruction).
+template <class T>
+__device__ __forceinline__ T kept(T v)
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("" : "+r"(v));
+#endif
+    return v;
+}
+
 // Bytes of shared memory by their 32-bit address there.  Pointers would do,
 // but the interpreter's loop selects between two of them and keeps several:
 // as generic pointers they cost 64-bit arithmetic.
@@ -295,6 +306,23 @@ inline const uint32_t* tia_table()
     return t.w;
 }
 #endif
+// The high half of a table word w: loaded again rather than shifted out (the
+// headless loop is bound by the ALU pipe, of which a shift is an instruction:
+// 50 and 45 of them a guest instruction, the mixed batch 14.1 and 13.8 ms);
+// the rendering loop is not, and shifts (load false).
+enum : uint32_t { H_CYC = 6u, H_LEN = 10u, H_M = 14u, H_K = 22u, H_X = 26u };
+template <bool LOAD>
+__device__ __forceinline__ uint32_t high(sptr tab, uint32_t op, uint32_t h, uint32_t w)
+{
+    if constexpr (!LOAD) return w >> 16;
+#ifdef __CUDA_ARCH__
+    uint32_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(tab + op * 32u + h));
+    return v;
+#else
+    return ((const uint32_t*)((const OpWord*)tab + op))[h / 4u] >> 16;
+#endif
+}
 __device__ __forceinline__ OpWord ldw(sptr tab, uint32_t op)
 {
 #ifdef __CUDA_ARCH__
@@ -934,35 +962,35 @@ static __device__ __noinline__ RRead render_io_read(uint32_t a, uint32_t owed, R
 // The DPC chip of FA_SCHEME_DPC carts (no counterpart in the reference),
 // with the semantics the oracle's DPC section fixes: 8 data fetchers (11-bit
 // counter, top, bottom, flag), an 8-bit random number generator and 3 music
-// channels clocked at 20 kHz of Cpu::cycles.  The registers stay in their
-// HBM rows (R_DPC_*) and are changed there in place, one access at a time:
-// a read of $1000-$103F (wr 0; returns the value) or a write of v to
-// $1040-$107F (wr 1).  cyc_acc: the instruction cycles not yet added to the
-// rows' Cpu::cycles (none of the accessing instruction's).  `disp` is the
-// 2K of display data.  One out-of-line copy for every access site.
+// channels clocked at 20 kHz of Cpu::cycles.  The registers are the R_DPC_*
+// rows from R_DPC_CNT on, register word k at d[k * S]: while a unit runs, in
+// the console's shared-memory slab (as rows of HBM, changed in place one
+// access at a time, they were 7 dependent loads, and the oscillator two 64-bit
+// divisions, an access).  A read of $1000-$103F (wr 0; returns the value) or
+// a write of v to $1040-$107F (wr 1).  now: the oscillator's clocks before the
+// accessing instruction.  `disp` is the 2K of display data.
 static __device__ __forceinline__ uint32_t dpc_byte(uint32_t w, uint32_t k) { return (w >> ((k & 3u) * 8u)) & 0xFFu; }
 
-static __device__ __forceinline__ uint32_t dpc_io(uint32_t a, uint32_t v, uint32_t wr, uint32_t* col, uint32_t S,
-                                               const uint8_t* disp, uint32_t cyc_acc)
+static __device__ __forceinline__ uint32_t dpc_io(uint32_t a, uint32_t v, uint32_t wr, uint32_t* d, uint32_t S, sptr disp,
+                                                  uint32_t now)
 {
-    const uint32_t misc = col[(size_t)R_DPC_MISC * S];
+    constexpr uint32_t CNT = 0u, TOP = R_DPC_TOP - R_DPC_CNT, BOT = R_DPC_BOT - R_DPC_CNT, MISC = R_DPC_MISC - R_DPC_CNT,
+                       OSC = R_DPC_OSC - R_DPC_CNT;
+    const uint32_t misc = d[MISC * S];
     uint32_t flags = misc & 0xFFu, music = (misc >> 8) & 7u, rnd = (misc >> 16) & 0xFFu;
     // The music channels up to the instruction's start: one clock of the
     // oscillator counts a channel's low byte down, the clock after 0 reloads
     // top; the flag is set while the low byte is above bottom.
-    const unsigned long long t =
-        (((unsigned long long)col[(size_t)R_CYC_HI * S] << 32) | col[(size_t)R_CYC_LO * S]) + cyc_acc;
-    const uint32_t now = (uint32_t)((t / 3579545ull) * 60000ull + ((t % 3579545ull) * 60000ull) / 3579545ull);
-    const uint32_t clocks = now - col[(size_t)R_DPC_OSC * S];
-    col[(size_t)R_DPC_OSC * S] = now;
+    const uint32_t clocks = now - d[OSC * S];
+    d[OSC * S] = now;
     if (clocks && music) {
 #pragma unroll 1
         for (uint32_t f = 5u; f < 8u; f++) {
             if (!((music >> (f - 5u)) & 1u)) continue;
-            uint32_t& cw = col[(size_t)(R_DPC_CNT + (f >> 1)) * S];
+            uint32_t& cw = d[(CNT + (f >> 1)) * S];
             const uint32_t sh = (f & 1u) * 16u, cnt = (cw >> sh) & 0x7FFu;
-            const uint32_t top = dpc_byte(col[(size_t)(R_DPC_TOP + (f >> 2)) * S], f);
-            const uint32_t bot = dpc_byte(col[(size_t)(R_DPC_BOT + (f >> 2)) * S], f);
+            const uint32_t top = dpc_byte(d[(TOP + (f >> 2)) * S], f);
+            const uint32_t bot = dpc_byte(d[(BOT + (f >> 2)) * S], f);
             uint32_t low = cnt & 0xFFu;
             low = clocks <= low ? low - clocks : top - (clocks - low - 1u) % (top + 1u);
             cw = (cw & ~(0xFFFFu << sh)) | (((cnt & 0x700u) | low) << sh);
@@ -970,9 +998,9 @@ static __device__ __forceinline__ uint32_t dpc_io(uint32_t a, uint32_t v, uint32
         }
     }
     const uint32_t k = a & 7u, f = (a >> 3) & 7u, sh = (k & 1u) * 16u;
-    uint32_t& cw = col[(size_t)(R_DPC_CNT + (k >> 1)) * S];
-    uint32_t& tw = col[(size_t)(R_DPC_TOP + (k >> 2)) * S];
-    uint32_t& bw = col[(size_t)(R_DPC_BOT + (k >> 2)) * S];
+    uint32_t& cw = d[(CNT + (k >> 1)) * S];
+    uint32_t& tw = d[(TOP + (k >> 2)) * S];
+    uint32_t& bw = d[(BOT + (k >> 2)) * S];
     uint32_t cnt = (cw >> sh) & 0x7FFu, out = 0u;
     if (!wr) {
         const bool mus = k >= 5u && ((music >> (k - 5u)) & 1u);
@@ -983,7 +1011,7 @@ static __device__ __forceinline__ uint32_t dpc_io(uint32_t a, uint32_t v, uint32
             if (low == dpc_byte(tw, k)) flags |= 1u << k;
             else if (low == dpc_byte(bw, k)) flags &= ~(1u << k);
         }
-        const uint32_t flag = ((flags >> k) & 1u) ? 0xFFu : 0u, data = disp[2047u - cnt];
+        const uint32_t flag = ((flags >> k) & 1u) ? 0xFFu : 0u, data = lds8(disp + (2047u - cnt));
         switch (f) {
         case 0:
             if (k < 4u) out = rnd;
@@ -1010,7 +1038,7 @@ static __device__ __forceinline__ uint32_t dpc_io(uint32_t a, uint32_t v, uint32
         default: break;
         }
     }
-    col[(size_t)R_DPC_MISC * S] = flags | (music << 8) | (rnd << 16);
+    d[MISC * S] = flags | (music << 8) | (rnd << 16);
     return out;
 }
 
@@ -1166,6 +1194,7 @@ struct Emu {
     uint32_t i;              // the instance's index in its group
     const uint8_t* rom;      // shared-memory ROM image, nbanks * 4 KiB
     uint32_t hot_lo, nbanks;
+    int32_t lim;             // 4K-bank carts: ROM addresses << 19 below this, and the next two, are clear of the hotspots
     // ---- CPU (src/cpu.rs:96-105)
     // P is kept apart: what an instruction sets costs one move or none, and
     // PHP, BRK and the state rows assemble it (get_p / set_p).
@@ -1321,7 +1350,70 @@ struct Emu {
     // DPC core: reads of $1000-$103F and writes of $1040-$107F reach the registers.
     __device__ __forceinline__ uint32_t dpc(uint32_t a13, uint32_t v, uint32_t wr)
     {
-        return dpc_io(a13, v, wr, column(), G->stride, rom + 8192u, cyc_acc + el);
+        return dpc_io(a13, v, wr, dpc_regs(), dpc_step(), to_sptr(rom) + 8192u, dpc_now());
+    }
+    // The DPC core's registers: FA_DPC_WORDS rows of BLOCK words after the
+    // RAM in the console's slab (the host runs on the rows of the column).
+    // The last two hold the oscillator at the frame's start: its clocks, and
+    // the remainder of the division.
+    __device__ __forceinline__ uint32_t* dpc_regs() const
+    {
+#ifdef __CUDA_ARCH__
+        const uint32_t t = threadIdx.x & (BLOCK - 1u);
+        return (uint32_t*)(pv - t + BLOCK * 128u) + t;
+#else
+        return &row(R_DPC_CNT);
+#endif
+    }
+    __device__ __forceinline__ uint32_t dpc_step() const
+    {
+#ifdef __CUDA_ARCH__
+        return BLOCK;
+#else
+        return G->stride;
+#endif
+    }
+    // The oscillator's clocks at the instruction's start, 60000 per 3579545
+    // of Cpu::cycles (as 12000 per 715909), exactly.
+    __device__ __forceinline__ uint32_t dpc_now() const
+    {
+        const uint32_t n = cyc_acc + el;
+#ifdef __CUDA_ARCH__
+        const uint32_t* d = dpc_regs();
+        const uint32_t q = d[(FA_DPC_WORDS - 2u) * BLOCK], r = d[(FA_DPC_WORDS - 1u) * BLOCK];
+        if (n < 350000u) return q + (r + n * 12000u) / 715909u;       // r < 715909: within 32 bits
+        return q + (uint32_t)((r + n * 12000ull) / 715909ull);
+#else
+        const uint2 b = dpc_clock();
+        return b.x + (uint32_t)((b.y + n * 12000ull) / 715909ull);
+#endif
+    }
+    __device__ __forceinline__ uint2 dpc_clock() const                // of the rows' Cpu::cycles
+    {
+        const unsigned long long t = ((unsigned long long)row(R_CYC_HI) << 32) | row(R_CYC_LO);
+        const unsigned long long x = (t % 715909ull) * 12000ull;
+        return make_uint2((uint32_t)(t / 715909ull * 12000ull + x / 715909ull), (uint32_t)(x % 715909ull));
+    }
+    // At a frame's start, after Cpu::cycles was brought up to date.
+    __device__ __forceinline__ void dpc_frame()
+    {
+#ifdef __CUDA_ARCH__
+        const uint2 b = dpc_clock();
+        dpc_regs()[(FA_DPC_WORDS - 2u) * BLOCK] = b.x;
+        dpc_regs()[(FA_DPC_WORDS - 1u) * BLOCK] = b.y;
+#endif
+    }
+    __device__ __forceinline__ void load_dpc()
+    {
+#ifdef __CUDA_ARCH__
+        for (uint32_t k = 0; k < FA_DPC_WORDS - 2u; k++) dpc_regs()[k * BLOCK] = row(R_DPC_CNT + k);
+#endif
+    }
+    __device__ __forceinline__ void store_dpc() const
+    {
+#ifdef __CUDA_ARCH__
+        for (uint32_t k = 0; k < FA_DPC_WORDS - 2u; k++) row(R_DPC_CNT + k) = dpc_regs()[k * BLOCK];
+#endif
     }
     // 3F: a write of v to $0000-$003F maps 2K bank v mod n at $1000-$17FF.
     __device__ __forceinline__ void f3_write(uint32_t a13, uint32_t v)
@@ -1632,7 +1724,7 @@ struct Emu {
         if constexpr (DPC) return a0 >= 0x1040u && (a0 & 0x3FFu) <= 0x3FDu && (a0 + 2u < 0x1FF8u || a0 > 0x1FF9u);
         else if constexpr (FE) return a0 >= 0x1000u && (a0 & 0x3FFu) <= 0x3FDu;
         else if constexpr (SLICED) return a0 >= 0x1000u && (a0 & 0x3FFu) <= 0x3FDu && (a0 + 2u < 0x1FE0u || a0 > 0x1FF7u);
-        else return (int32_t)(pc << 19) < (int32_t)((hot_lo - 2u) << 19);   // ROM addresses are negative, in order
+        else return (int32_t)(pc << 19) < lim;   // ROM addresses are negative, in order
     }
     // ROM data at ea, below every hotspot: a load without a side effect
     // (wr, T_WR or 0: and no write).
@@ -1642,7 +1734,7 @@ struct Emu {
         if constexpr (DPC) return (uint32_t)s - (0x1040u << 19) < ((0x1FF8u - 0x1040u) << 19);
         else if constexpr (FE) return s < 0;
         else if constexpr (SLICED) return s < (int32_t)(0x1FE0u << 19);
-        else return s < (int32_t)(hot_lo << 19);                         // Fixed: hot_lo $2000, all of it
+        else return s < lim;
     }
     __device__ __forceinline__ uint32_t rom_at(uint32_t a) const { return SLICED ? srom(a) : bank | (a & 0xFFFu); }
 
@@ -1672,7 +1764,8 @@ struct Emu {
     template <class LOOK>
     __device__ __forceinline__ uint32_t run(uint32_t wait_key, LOOK look)
     {
-        const sptr tab = to_sptr(op_table()), rs = to_sptr(rom), ps = to_sptr(pv);
+        const sptr tab = to_sptr(op_table()), rs = RENDER ? to_sptr(rom) : kept(to_sptr(rom)),
+                   ps = RENDER ? to_sptr(pv) : kept(to_sptr(pv));
         uint32_t n;
         const uint32_t end = instr + FA_BURST;
 #pragma unroll 1
@@ -1688,9 +1781,9 @@ struct Emu {
             const uint32_t b1 = lds8(q + 1), b2 = lds8(q + 2);
             OpWord w = ldw(tab, op);
             const uint32_t f = w.ix;
-            const uint32_t pc1 = pc + (w.rd >> 16);                   // past $FFFF: not ok, and exec() masks it
+            const uint32_t pc1 = pc + high<!RENDER>(tab, op, H_LEN, w.rd);            // past $FFFF: not ok, and exec() masks it
             uint32_t base = __byte_perm(b1, b2, w.bs);
-            n = w.rs >> 16;
+            n = high<!RENDER>(tab, op, H_CYC, w.rs);
             if (!ok | ((f & T_CTRL) != 0u)) {
                 if (!ok) goto exec_;
                 if (f & T_BR) {
@@ -1774,6 +1867,8 @@ struct Emu {
                 const bool ram = ((ea & 0x1E80u) == 0x80u) & !(FE && (ea & 0x1FFFu) == 0x1FEu);
                 const sptr pr = ps + poff(ea & 0x7Fu), po = rs + rom_at(ea);
                 uint32_t ld = lds8(ram ? pr : po);
+                uint32_t wm = high<!RENDER>(tab, op, H_M, w.bs), wk = high<!RENDER>(tab, op, H_K, w.fs),
+                         wx = high<!RENDER>(tab, op, H_X, w.am);
                 const bool plain = ram | data_ok(ea, f);
                 const bool far = ((base ^ ea) & 0xFF00u) != 0u;       // a page crossed
                 if (!plain | far | ((f & (pd | (T_ODD | T_FIX))) != 0u)) {
@@ -1803,19 +1898,25 @@ struct Emu {
                             }
                         }
                         if (!RENDER && (a & 0x1287u) == 0x284u && !intim_quick()) goto exec_;
-                        if (!wr | rmw) {
+                        // A DPC register: a read of $1000-$103F or a write to $1040-$107F.
+                        if (DPC && rmw && a - 0x1000u < 0x80u) goto exec_;
+                        const bool reg = DPC && a - 0x1000u - (wr ? 0x40u : 0u) < 0x40u;
+                        if (reg) {
+                            ld = dpc(a, __byte_perm(R, 0u, w.rs), wr ? 1u : 0u);
+                            if (wr) { pc = pc1; goto done_; }
+                        } else if (!wr | rmw) {
                             const uint32_t j = n - (rmw ? 3u : 1u);
                             if (a & 0x1000u) {
                                 hot(a);
-                                ld = (DPC && a < 0x1040u) ? dpc(a, 0u, 0u) : lds8(rs + rom_at(ea));
+                                ld = lds8(rs + rom_at(ea));
                             } else {
                                 ld = bus_read(a, j);
                             }
                         }
                         if (wr) {
-                            uint32_t r = alu(w, ld, b1);
+                            uint32_t r = __byte_perm(R, 0u, w.rs);
                             if (rmw) {
-                                if (f & T_ODD) r = shift(w, o, ld);
+                                r = (f & T_ODD) ? shift(w, o, ld) : alu(w, ld, b1);
                                 F = __byte_perm(F, r, (f & T_ODD) ? 0x3574u : w.fs);
                             }
 #pragma unroll 1
@@ -1823,7 +1924,6 @@ struct Emu {
                                 const uint32_t u = (m ? r : ld) & 0xFFu;
                                 if (a & 0x1000u) {
                                     hot(a);
-                                    if (DPC && a - 0x1040u < 0x40u) (void)dpc(a, u, 1u);
                                 } else {
                                     bus_write(a, u, n - 2u + m);
                                 }
@@ -1832,13 +1932,17 @@ struct Emu {
                             goto done_;
                         }
                     }
+                    if constexpr (RENDER) {                           // not kept in registers across the pixel code's calls
+                        w = ldw(tab, op);
+                        wm = w.bs >> 16; wk = w.fs >> 16; wx = w.am >> 16;
+                    }
                     if (f & (pd | T_ODD)) {
                         odd_op(w, o, ld, b1, pr, wr);
                         wr = false;
                         w.rd = w.fs = 0x3210u;                        // completed: nothing changes below
                     }
                 }
-                const uint32_t r = alu(w, ld, b1);
+                const uint32_t r = alu(w, ld, b1, wm, wk, wx);
                 if (wr) sts8(pr, r);
                 commit(w, r);
                 pc = pc1;
@@ -1865,15 +1969,19 @@ struct Emu {
     }
 
     // The result of a table word's operation (byte 0), its carry (byte 1) and
-    // its V (bit 7 of byte 2): (s ^ v) + m (s & v) + q, with s ^ v left out for
-    // AND.  m = 2 adds (SBC and compares an inverted v), 1 ORs, 0 XORs; s = 0
-    // loads, v = 0 moves.
+    // its V (bit 7 of byte 2): k (s ^ v) + m (s & v) + q.  k is 1 but for AND;
+    // m = 2 adds (SBC and compares a v that x inverts), 1 ORs and ANDs, 0 XORs;
+    // s = 0 loads, v = 0 moves.  Multiplies: the ALU pipe is the busy one.
+    __device__ __forceinline__ uint32_t alu(const OpWord& w, uint32_t ld, uint32_t b1, uint32_t m, uint32_t k, uint32_t x) const
+    {
+        const uint32_t s = __byte_perm(R, 0u, w.rs), v = __byte_perm(ld, b1, w.xs) ^ x;
+        const uint32_t q = __byte_perm(F, 0xFF01u, w.qs);
+        const uint32_t r = (s & v) * m + ((s ^ v) * k + q);
+        return __byte_perm(r, (s ^ r) & (v ^ r), 0x3410u);
+    }
     __device__ __forceinline__ uint32_t alu(const OpWord& w, uint32_t ld, uint32_t b1) const
     {
-        const uint32_t s = __byte_perm(R, 0u, w.rs), v = __byte_perm(ld, b1, w.xs) ^ (w.am >> 16);
-        const uint32_t q = __byte_perm(F, 0xFF01u, w.qs);
-        const uint32_t r = ((s ^ v) & (uint32_t)((int32_t)w.qs >> 31)) + q + (s & v) * (w.bs >> 16);
-        return __byte_perm(r, (s ^ r) & (v ^ r), 0x3410u);
+        return alu(w, ld, b1, w.bs >> 16, w.fs >> 16, w.am >> 16);
     }
     __device__ __forceinline__ void commit(const OpWord& w, uint32_t r)
     {
@@ -1965,6 +2073,12 @@ struct Emu {
         if constexpr (!RENDER) {
             if (!(a & 0x200u)) {
                 const uint32_t r = a & 0x3Fu, e = tia_table()[r];
+                if (r == 2u) {                                        // WSYNC: the frame loop looks
+                    if constexpr (SLICED) f3_write(a, v);
+                    tw |= TW_WSYNC;
+                    dl = 0;
+                    return;
+                }
                 if (e) {                                              // a register that only keeps bits of v
                     if constexpr (SLICED) f3_write(a, v);
                     ((uint8_t*)column())[cold_off(e & 0xFFu, grp()->stride * 4u)] = (uint8_t)((v >> ((e >> 8) & 0xFFu)) & (e >> 16));
@@ -2252,6 +2366,7 @@ struct Emu {
         tp = col[R_TIMER * stride];
         w = col[R_SELPC * stride]; su = (w & 0xFFFFu) | (((p1 >> 16) & 0xFFu) << 16); pcnt = w >> 16;
         tlim = RENDER ? 0u : pia_span();
+        lim = kept((int32_t)((hot_lo - 2u) << 19));
         w = col[R_TIA0 * stride];  clock = w & 0xFFFF; scanline = w >> 16;
         w = col[R_TIA1 * stride];                                   // wsync fcomp vsync vblank
         tw = ((w >> 16) & 0xFFFFu) | ((w & 1u) << 16) | (((w >> 8) & 1u) << 17) | (((p1 >> 24) & 1u) << 18);

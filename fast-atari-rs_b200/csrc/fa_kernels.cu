@@ -61,7 +61,7 @@ static bool warp_layout(FaLaunch& L, int block, bool persistent, int* warps)
 {
     const uint32_t lib = plan_romlib(L);
     L.romlib_bytes = lib;
-    const uint32_t slab = FA_SMEM_WORDS * 32u * 4u;
+    const uint32_t slab = fa_slab_words(fa_maps_of(L.g, L.ngroups)) * 32u * 4u;
     const int fit = (int)((FA_SMEM_PER_CTA_MAX - (int)lib) / (int)slab);
     if (fit < block / 32) return false;
     int w = block / 32;
@@ -127,7 +127,7 @@ cudaError_t fa_launch_prepare(const FaLaunch& L, int block, bool persistent)
 
 int fa_launch_occupancy(int block, uint32_t rom_bytes_max)
 {
-    const size_t base = (size_t)rom_bytes_max + (size_t)FA_SMEM_WORDS * block * 4u;
+    const size_t base = (size_t)rom_bytes_max + (size_t)fa_slab_words(FA_MAPS_4K) * block * 4u;
     return FaCore<FA_MAPS_4K>::occupancy(block, base);
 }
 

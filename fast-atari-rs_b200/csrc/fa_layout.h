@@ -19,6 +19,9 @@
 // registers (rows FA_SMEM_WORDS..FA_PRIV_WORDS-1) stay in their HBM rows and
 // are touched there by the rare TIA register writes and collision reads.
 #define FA_SMEM_WORDS 32
+// The DPC core keeps its registers beside it (Emu::dpc_regs): the R_DPC_*
+// rows, and the oscillator at the frame's start.
+#define FA_DPC_WORDS 12u
 
 // Private-byte offsets: RAM occupies [0, 128).
 enum : uint32_t {
@@ -101,6 +104,11 @@ FA_HD static inline uint32_t fa_map_kind(uint32_t hot_lo) { return hot_lo < 0x10
 // Kernel builds by the cores they hold (see run_unit): 4K-bank carts only,
 // several kinds, E0 / 3F carts only, DPC carts only, FE carts only.
 enum : int { FA_MAPS_4K = 0, FA_MAPS_BOTH = 1, FA_MAPS_SLICED = 2, FA_MAPS_DPC = 3, FA_MAPS_FE = 4 };
+// Shared-memory words a console takes in a build.
+FA_HD static constexpr uint32_t fa_slab_words(int maps)
+{
+    return FA_SMEM_WORDS + (maps == FA_MAPS_DPC || maps == FA_MAPS_BOTH ? FA_DPC_WORDS : 0u);
+}
 
 // E0 and 3F; the 4K-bank pair of DPC and FE (bank b: slices 4b..4b+3, FE's
 // armed flag in bit 7); any scheme.  Each device core calls only its own.

@@ -122,7 +122,9 @@ struct Runner {
             for (uint32_t w = FA_SMEM_WORDS; w < (DPC ? (uint32_t)FA_ROWS : (uint32_t)R_DPC_CNT); w++)
                 e.row(w) = G->snapshot[w];
             e.load_hot(G->snapshot, 1);
+            if constexpr (DPC) e.load_dpc();
         }
+        if constexpr (DPC) e.dpc_frame();
         if (G->actions) e.apply_action(G->actions[(size_t)f * G->act_stride + e.i]);
         if (e.row(R_STATUS) & FA_STATUS_HALT_MASK) return false;
         e.tw &= ~TW_FCOMP;
@@ -148,7 +150,25 @@ struct Runner {
     // started, as a run_one_cycle of its own.
     __device__ __forceinline__ void attend(uint32_t n)
     {
+        if (e.wsync()) {
+            // A wait with nothing else due, on the line of the last sync: the
+            // usual STA WSYNC.  Its instruction and the wait in one piece.
+            const uint32_t c = e.clock + 3u * e.el, wait = (230u - c) / 3u, all = e.el + wait;
+            if ((c < 228u) & (e.scanline < 262u) & (phase != 0u) & !e.vsync_on() & (all < e.tlim) &
+                (e.cyc_acc + fcyc + all <= FA_FRAME_CYCLE_CAP)) {
+                e.tlim -= all;
+                e.cyc_acc += e.el;
+                fcyc += wait;
+                e.el = 0;
+                e.clock = 228u;
+                e.end_scanline();
+                e.dl = due();
+                return;
+            }
+        }
+        const uint32_t set = e.tw & TW_WSYNC;                         // by this instruction: not one of the folded lines clears it
         e.fold(e.el - n);
+        e.tw |= set;
         e.el = 0;
         if (n) {
             e.tia_tick(n);
@@ -326,6 +346,7 @@ __device__ __forceinline__ void run_unit_as(const FaGroup& G, uint32_t first, ui
     if (valid) {
         r.e.load_ram(col, G.stride);
         r.e.load_hot(col, G.stride);
+        if constexpr (DPC) r.e.load_dpc();
         if (G.k > 0) r.active = r.begin_frame();
     }
     const uint32_t rounds = run_lanes(r, G.sched);
@@ -337,6 +358,7 @@ __device__ __forceinline__ void run_unit_as(const FaGroup& G, uint32_t first, ui
             r.e.apply_action(G.actions[(size_t)(G.k - 1u) * G.act_stride + r.e.i]);
         r.e.store_ram(col, G.stride);
         r.e.store_hot(col, G.stride);
+        if constexpr (DPC) r.e.store_dpc();
         if (G.obs) {
             uint4* o = (uint4*)(G.obs + (size_t)r.e.i * 128u);
 #pragma unroll 2
