@@ -465,7 +465,6 @@ struct RState {
     uint32_t rx;                                // the current line's pixels are drawn up to this clock
     uint32_t sc;                                // the framebuffer sector (32 pixels) whose pixels the sector buffer holds
     uint32_t zr;                                // rows written since the clear point | R_ZPEND (rows after them not yet zeroed)
-    uint32_t tv, ps, sel, uf;                   // PIA timer
 };
 constexpr uint32_t R_ZPEND = 0x100u;
 
@@ -754,40 +753,37 @@ static __device__ __noinline__ RState render_observe(RState s, uint8_t* pv, uint
     return s;
 }
 
-static __device__ __forceinline__ void r_pia_tick(RState& s)     // pia.rs:80-103
+// The PIA timer of the rendering console: value | prescaler << 16, interval |
+// underflow << 16.
+static __device__ __forceinline__ void r_pia_tick(uint32_t& tv, uint32_t& ps, uint32_t sel, uint32_t& uf)     // pia.rs:80-103
 {
-    if (s.tv == 0 && s.uf) { s.tv = 0xFFu; return; }
-    s.ps = (s.ps - 1u) & 0xFFFFu;
-    if (s.ps == 0) {
-        s.ps = s.uf ? 1u : s.sel;
-        if (s.tv == 0) { s.uf = 1; s.tv = 0xFFu; } else s.tv -= 1u;
+    if (tv == 0 && uf) { tv = 0xFFu; return; }
+    ps = (ps - 1u) & 0xFFFFu;
+    if (ps == 0) {
+        ps = uf ? 1u : sel;
+        if (tv == 0) { uf = 1; tv = 0xFFu; } else tv -= 1u;
     }
 }
 
-// m calls of Pia::tick (pia.rs:80-103), a prescaler period at a time.
-static __device__ __forceinline__ void r_pia_ticks(RState& s, uint32_t m)
+// m calls of Pia::tick (pia.rs:80-103), a prescaler period at a time.  Only
+// the accesses that see or set the timer, and the state's store, need them:
+// the TIA and the PIA do not interact.
+static __device__ __noinline__ uint2 r_pia_ticks(uint32_t tp, uint32_t su, uint32_t m)
 {
+    uint32_t tv = tp & 0xFFFFu, ps = tp >> 16, sel = su & 0xFFFFu, uf = su >> 16;
     while (m) {
-        if (s.ps == 0 || (s.uf && s.tv == 0)) { r_pia_tick(s); m--; continue; }
-        if (s.uf && s.ps == 1u) { s.tv = (s.tv - m) & 0xFFu; return; }   // after underflow: one count per tick
-        if (m < s.ps) { s.ps -= m; return; }
-        m -= s.ps;                                                   // the tick that empties the prescaler
-        s.ps = s.uf ? 1u : s.sel;
-        if (s.tv == 0) { s.uf = 1; s.tv = 0xFFu; } else s.tv -= 1u;
+        if (ps == 0 || (uf && tv == 0)) { r_pia_tick(tv, ps, sel, uf); m--; continue; }
+        if (uf && ps == 1u) { tv = (tv - m) & 0xFFu; break; }         // after underflow: one count per tick
+        if (m < ps) { ps -= m; break; }
+        m -= ps;                                                     // the tick that empties the prescaler
+        ps = uf ? 1u : sel;
+        if (tv == 0) { uf = 1; tv = 0xFFu; } else tv -= 1u;
     }
+    return make_uint2(tv | (ps << 16), sel | (uf << 16));
 }
 
-// n CPU cycles of the rendering console: three TIA clocks and one PIA clock
-// each (the TIA and the PIA do not interact, so each is advanced in bulk).
-static __device__ __noinline__ RState render_cycles(RState s, uint32_t n, uint32_t pins, uint8_t* pv, uint8_t* fbp)
-{
-    r_advance(s, 3u * n, pins, pv, fbp);
-    r_pia_ticks(s, n);
-    return s;
-}
-
-// n TIA clocks alone (the clocks around a PIA write, src/atari.rs:207-222).
-static __device__ __noinline__ RState render_tia_ticks(RState s, uint32_t n, uint32_t pins, uint8_t* pv, uint8_t* fbp)
+// n TIA clocks.
+static __device__ __noinline__ RState render_clocks(RState s, uint32_t n, uint32_t pins, uint8_t* pv, uint8_t* fbp)
 {
     r_advance(s, n, pins, pv, fbp);
     return s;
@@ -887,48 +883,29 @@ static __device__ __forceinline__ void r_write(uint32_t a, uint32_t v, RState& s
     }
 }
 
-// `owed` whole CPU cycles, then Bus::write of a TIA register
-// (src/atari.rs:207-222): two TIA clocks, the write, one TIA clock and the
-// PIA clock.  One call per write: the cycles before it ride along.
-static __device__ __noinline__ RState render_write_cycle(uint32_t a, uint32_t v, uint32_t owed, RState s, uint32_t pins,
-                                                         uint8_t* pv, uint8_t* fbp)
+// `n` TIA clocks (those owed and the two of its own cycle before the write,
+// src/atari.rs:207-222), then the write of a TIA register.  The clock after
+// it is owed with the cycles that follow.
+static __device__ __noinline__ RState render_write(uint32_t a, uint32_t v, uint32_t n, RState s, uint32_t pins, uint8_t* pv,
+                                                   uint8_t* fbp)
 {
-    if (owed) {
-        r_advance(s, 3u * owed, pins, pv, fbp);
-        r_pia_ticks(s, owed);
-    }
-    r_advance(s, 2u, pins, pv, fbp);
+    r_advance(s, n, pins, pv, fbp);
     r_write(a, v, s, pv, fbp);
-    r_advance(s, 1u, pins, pv, fbp);
-    r_pia_tick(s);
     return s;
 }
 
-// Tia::read (tia.rs:533-566) or Pia::read of an I/O register (pia.rs:169-199);
-// .y = 1 when the read clears the timer's underflow flag (INTIM).
-static __device__ __forceinline__ uint2 r_read_value(uint32_t a, const RState& s, uint32_t pins, uint32_t pads,
-                                                     uint32_t ports, const uint8_t* pv)
+// Tia::read (tia.rs:533-566).
+static __device__ __forceinline__ uint32_t r_read_tia(uint32_t a, const RState& s, uint32_t pins, uint32_t pads, const uint8_t* pv)
 {
-    if ((a & 0x1080u) == 0) {
-        const uint32_t r = a & 0x0Fu;
-        if (r < 8u) return make_uint2(rp8(pv, PB_CX + r), 0u);
-        switch (r) {
-        case 0x8: return make_uint2(s.pcnt >= (pads & 0xFFu) ? 0x80u : 0u, 0u);
-        case 0x9: return make_uint2(s.pcnt >= ((pads >> 8) & 0xFFu) ? 0x80u : 0u, 0u);
-        case 0xA: case 0xB: return make_uint2(0x80u, 0u);
-        case 0xC: return make_uint2((s.tw & TW_LATCH) ? ((s.tw & TW_L4) ? 0x80u : 0u) : ((pins & 0x10000u) ? 0x80u : 0u), 0u);
-        case 0xD: return make_uint2((s.tw & TW_LATCH) ? ((s.tw & TW_L5) ? 0x80u : 0u) : ((pins & 0x20000u) ? 0x80u : 0u), 0u);
-        default: return make_uint2(0u, 0u);
-        }
-    }
-    switch (a & 7u) {
-    case 0: { const uint32_t ddr = (ports >> 8) & 0xFFu; return make_uint2(((pins & 0xFFu) & ~ddr) | (ports & ddr & 0xFFu), 0u); }
-    case 1: return make_uint2((ports >> 8) & 0xFFu, 0u);
-    case 2: { const uint32_t ddr = ports >> 24; return make_uint2((((pins >> 8) & 0xFFu) & ~ddr) | ((ports >> 16) & ddr & 0xFFu), 0u); }
-    case 3: return make_uint2(ports >> 24, 0u);
-    case 4: return make_uint2(s.tv & 0xFFu, 1u);
-    case 5: return make_uint2(s.uf ? 0x80u : 0u, 0u);
-    default: return make_uint2(0u, 0u);
+    const uint32_t r = a & 0x0Fu;
+    if (r < 8u) return rp8(pv, PB_CX + r);
+    switch (r) {
+    case 0x8: return s.pcnt >= (pads & 0xFFu) ? 0x80u : 0u;
+    case 0x9: return s.pcnt >= ((pads >> 8) & 0xFFu) ? 0x80u : 0u;
+    case 0xA: case 0xB: return 0x80u;
+    case 0xC: return (s.tw & TW_LATCH) ? ((s.tw & TW_L4) ? 0x80u : 0u) : ((pins & 0x10000u) ? 0x80u : 0u);
+    case 0xD: return (s.tw & TW_LATCH) ? ((s.tw & TW_L5) ? 0x80u : 0u) : ((pins & 0x20000u) ? 0x80u : 0u);
+    default: return 0u;
     }
 }
 
@@ -937,24 +914,17 @@ struct RRead {
     uint32_t v;
 };
 
-// `owed` whole CPU cycles, then the read of a TIA or PIA register in its own
-// cycle (Bus::read, src/atari.rs:195-205): collisions drawn up to the beam,
-// the value, then three TIA clocks and the PIA clock.  One call per read.
-static __device__ __noinline__ RRead render_io_read(uint32_t a, uint32_t owed, RState s, uint32_t pins, uint32_t pads,
-                                                    uint32_t ports, uint8_t* pv, uint8_t* fbp)
+// `n` owed TIA clocks, then the read of a TIA register (Bus::read,
+// src/atari.rs:195-205), collisions drawn up to the beam.  The clocks of its
+// own cycle are owed with those that follow.
+static __device__ __noinline__ RRead render_read(uint32_t a, uint32_t n, RState s, uint32_t pins, uint32_t pads, uint8_t* pv,
+                                                 uint8_t* fbp)
 {
-    if (owed) {
-        r_advance(s, 3u * owed, pins, pv, fbp);
-        r_pia_ticks(s, owed);
-    }
-    if ((a & 0x1080u) == 0 && (a & 0x0Fu) < 8u) r_pending(s, pv, fbp, s.clock);   // collisions so far
-    const uint2 r = r_read_value(a, s, pins, pads, ports, pv);
-    if (r.y) s.uf = 0;                                               // INTIM read clears the flag
-    r_advance(s, 3u, pins, pv, fbp);
-    r_pia_tick(s);
+    r_advance(s, n, pins, pv, fbp);
+    if ((a & 0x0Fu) < 8u) r_pending(s, pv, fbp, s.clock);            // collisions so far
     RRead out;
+    out.v = r_read_tia(a, s, pins, pads, pv);
     out.s = s;
-    out.v = r.x;
     return out;
 }
 
@@ -1551,11 +1521,23 @@ struct Emu {
     __device__ __forceinline__ uint32_t io(uint32_t a, uint32_t j)   // TIA or PIA register read
     {
         if constexpr (RENDER) {
-            const uint32_t d = lag + j;                               // cycles owed before this one
-            const RRead r = render_io_read(a, (int32_t)d > 0 ? d : 0u, rpack(), pins, pads, ports, pv, fbp);
-            runpack(r.s);
-            lag = 0u - (j + 1u);
-            return r.v;
+            if ((a & 0x1080u) == 0u) {
+                const RRead r = render_read(a, 3u * (lag + j) + tl, rpack(), pins, pads, pv, fbp);
+                runpack(r.s);
+                lag = 0u - j;
+                tl = 0;
+                return r.v;
+            }
+            const uint32_t k = a & 7u;                                // Pia::read (pia.rs:169-199)
+            if (k < 4u) {
+                const uint32_t od = ports >> ((k & 2u) * 8u), ddr = (od >> 8) & 0xFFu, in = pins >> ((k & 2u) * 4u);
+                return (k & 1u) ? ddr : ((in & ~ddr) | (od & ddr)) & 0xFFu;
+            }
+            if (k > 5u) return 0u;
+            pia_to(j);
+            if (k == 5u) return su >= 0x10000u ? 0x80u : 0u;
+            su &= 0xFFFFu;                                            // an INTIM read clears the underflow flag
+            return tp & 0xFFu;
         } else {
             if ((a & 0x87u) == 0x84u) {                             // INTIM: settles and clears the flag
                 intim();
@@ -1570,14 +1552,16 @@ struct Emu {
         if constexpr (SLICED) f3_write(a, v);                       // the write still reaches the TIA
         if constexpr (RENDER) {
             if ((a & 0x1080u) != 0) {                                 // PIA register: rare, the general path
-                rsync(j);
-                r_write_cycle(a, v);
+                pia_to(j);
+                const uint4 q = pia_write_io(a, v, ports, tp & 0xFFFFu, tp >> 16, su);
+                ports = q.x; tp = q.y | (q.z << 16); su = q.w;
             } else {
-                const uint32_t d = lag + j, t0 = tw;
-                runpack(render_write_cycle(a, v, (int32_t)d > 0 ? d : 0u, rpack(), pins, pv, fbp));
+                const uint32_t t0 = tw;
+                runpack(render_write(a, v, 3u * (lag + j) + tl + 2u, rpack(), pins, pv, fbp));
+                lag = 0u - (j + 1u);
+                tl = 1;
                 if (((tw ^ t0) & 0xFFu) || wsync()) done = 0;         // VSYNC changed, or a wait: the frame loop looks
             }
-            lag = 0u - (j + 1u);
         } else {
             sync();
             if (a & 0x200u) {
@@ -1957,6 +1941,7 @@ struct Emu {
             instr++;
             if constexpr (RENDER) {
                 lag += n;
+                plag += n;
                 cyc_acc += n;
             } else {
                 el += n;
@@ -2258,8 +2243,10 @@ struct Emu {
     // below), on the state they touch passed by value: one copy of the pixel
     // pipeline however many bus-access sites the interpreter has.
     uint32_t done;            // instruction cycles of the frame (cyc_acc) at which the frame loop must look
-    uint32_t lag;             // CPU cycles not yet given to the TIA and PIA; within an instruction, up to its start
+    uint32_t lag;             // CPU cycles not yet given to the TIA; within an instruction, up to its start
                              // (negative: they have reached cycle -lag of it)
+    uint32_t tl;              // and TIA clocks (0 or 1: the one after a register write) before those
+    uint32_t plag;            // CPU cycles not yet given to the PIA, likewise
     uint32_t vtop;            // visible_top | vblank_top << 16
     uint8_t* fbp;             // this instance's framebuffer, 160 x 192 palette indices
     uint32_t sc, zr;          // framebuffer sector in the sector buffer; rows written since the clear point | R_ZPEND
@@ -2269,61 +2256,40 @@ struct Emu {
     {
         RState r;
         r.clock = clock; r.scanline = scanline; r.tw = tw; r.pcnt = pcnt; r.vtop = vtop;
-        r.sc = sc; r.zr = zr; r.tv = tp & 0xFFFFu; r.ps = tp >> 16; r.sel = su & 0xFFFFu; r.uf = su >> 16;
-        r.rx = rx;
+        r.sc = sc; r.zr = zr; r.rx = rx;
         return r;
     }
     __device__ __forceinline__ void runpack(const RState& r)
     {
         clock = r.clock; scanline = r.scanline; tw = r.tw; pcnt = r.pcnt; vtop = r.vtop;
-        sc = r.sc; zr = r.zr; tp = r.tv | (r.ps << 16); su = r.sel | (r.uf << 16);
-        rx = r.rx;
+        sc = r.sc; zr = r.zr; rx = r.rx;
     }
-    // The TIA and the PIA up to cycle j of the current instruction.  They are
-    // advanced only before an access that observes or changes them: the
-    // cycles of instructions that touch only ROM and RAM are owed (lag) and
-    // given in one piece.
-    __device__ __forceinline__ void rsync(uint32_t j)
+    // The TIA is advanced only before an access that observes or changes it:
+    // the cycles of instructions that touch only ROM and RAM are owed (lag)
+    // and given in one piece, with the clocks of the access before.  So is the
+    // PIA, before the accesses that see or set its timer.
+    __device__ __forceinline__ void rcycles(uint32_t n)              // of a WSYNC wait, nothing owed
     {
-        const uint32_t d = lag + j;
-        if ((int32_t)d > 0) { runpack(render_cycles(rpack(), d, pins, pv, fbp)); lag = 0u - j; }
+        runpack(render_clocks(rpack(), 3u * n, pins, pv, fbp));
+        plag += n;
     }
-    __device__ __forceinline__ void rcycles(uint32_t n) { runpack(render_cycles(rpack(), n, pins, pv, fbp)); }
     __device__ __forceinline__ void settle()
     {
-        if (lag) { runpack(render_cycles(rpack(), lag, pins, pv, fbp)); lag = 0; }
+        const uint32_t n = 3u * lag + tl;
+        if (n) { runpack(render_clocks(rpack(), n, pins, pv, fbp)); lag = 0; tl = 0; }
     }
-    // Bus::write of a PIA register (src/atari.rs:207-222): two TIA clocks, the
-    // write, one TIA clock, the PIA clock.
-    __device__ __forceinline__ void r_write_cycle(uint32_t a, uint32_t v)
+    __device__ __forceinline__ void pia_to(uint32_t j)               // the PIA up to cycle j of the instruction
     {
-        RState r = render_tia_ticks(rpack(), 2u, pins, pv, fbp);
-        const uint4 q = pia_write_io(a, v, ports, r.tv, r.ps, r.sel | (r.uf << 16));
-        ports = q.x; r.tv = q.y; r.ps = q.z; r.sel = q.w & 0xFFFFu; r.uf = q.w >> 16;
-        r = render_tia_ticks(r, 1u, pins, pv, fbp);
-        runpack(r);
-        pia_tick1();
-    }
-    __device__ __forceinline__ void pia_tick1()                      // pia.rs:80-103
-    {
-        uint32_t tv = tp & 0xFFFFu, ps = tp >> 16, uf = su >> 16;
-        if (tv == 0 && uf) {
-            tv = 0xFFu;
-        } else {
-            ps = (ps - 1u) & 0xFFFFu;
-            if (ps == 0) {
-                ps = uf ? 1u : (su & 0xFFFFu);
-                if (tv == 0) { uf = 1; tv = 0xFFu; } else tv -= 1u;
-            }
-        }
-        tp = tv | (ps << 16);
-        su = (su & 0xFFFFu) | (uf << 16);
+        const uint2 r = r_pia_ticks(tp, su, plag + j);
+        tp = r.x; su = r.y;
+        plag = 0u - j;
     }
     // The owed cycles, the pixels up to the beam, and the framebuffer as it
     // can be seen now (the end of a frame or of a call).
     __device__ __forceinline__ void fb_observe()
     {
         settle();
+        pia_to(0u);
         runpack(render_observe(rpack(), pv, fbp));
     }
     // The sector buffer at the start of a call: the sector where the beam's
@@ -2359,7 +2325,7 @@ struct Emu {
         uint32_t w;
         R = col[R_AXYS * stride];
         w = col[R_PC * stride];    pc = w & 0xFFFF; set_p((w >> 16) & 0xFF); bank = (w >> 24) << 12;
-        cyc_acc = 0; el = 0;
+        cyc_acc = 0; el = 0; tl = 0; plag = 0;
         const uint32_t p0 = col[R_PIA0 * stride];                  // pa_out pa_ddr pa_in pb_out
         const uint32_t p1 = col[R_PIA1 * stride];                  // pb_ddr pb_in uf pdump
         ports = (p0 & 0xFFFFu) | ((p0 >> 24) << 16) | ((p1 & 0xFFu) << 24);

@@ -102,6 +102,7 @@ struct RRunner {
             // and PIA) before it stopped (src/cpu.rs:1139-1141): the TIA and
             // PIA are owed up to the end of that cycle.
             e.lag += 1u;
+            e.plag += 1u;
             e.fold_cycles();
             e.set_status(FA_STATUS_ILLEGAL_OPCODE);
             active = false;
