@@ -18,6 +18,8 @@
 // Dynamic shared memory a CTA may use (227 KiB opt-in limit minus the static
 // opcode table, barrier word and headroom).
 #define FA_SMEM_PER_CTA_MAX (227 * 1024 - 8192 - 1024)
+// Shared memory of an SM.
+#define FA_SMEM_PER_SM (228u * 1024u)
 
 // One cart's instance set in a launch.
 struct FaGroup {
@@ -55,7 +57,7 @@ struct FaLaunch {
     uint32_t nunits;
     uint32_t rom_bytes_max;      // shared-memory ROM bytes reserved per CTA (CTA-granular form)
     uint32_t romlib_bytes;       // all ROMs of the launch (warp-granular form, set by fa_launch_run)
-    uint32_t cta_warps;          // persistent form: warps per CTA cap (0 = as many as fit)
+    uint32_t cta_warps;          // persistent form: warps per CTA cap (0: by the carts and units)
     uint32_t* queue;             // work-queue counter (persistent form) or null
     uint32_t* err;               // device error word
     unsigned long long* instr;   // guest-instruction counter, or null
@@ -146,7 +148,7 @@ cudaError_t fa_launch_serve(const FaServeLaunch& L, int block, cudaStream_t s);
 cudaError_t fa_launch_run(const FaLaunch& L, int block, bool persistent, int sms, cudaStream_t s);
 // Everything fa_launch_run does before launching (kernel choice, shared-memory
 // attribute, occupancy), so that a later launch is safe inside a capture.
-cudaError_t fa_launch_prepare(const FaLaunch& L, int block, bool persistent);
+cudaError_t fa_launch_prepare(const FaLaunch& L, int block, bool persistent, int sms);
 // CTAs of fa_run<block> resident per SM for this ROM size (-1 on error).
 int fa_launch_occupancy(int block, uint32_t rom_bytes_max);
 cudaError_t fa_launch_broadcast(uint32_t* state, uint32_t stride, uint32_t n, const uint32_t* col,

@@ -54,55 +54,85 @@ static void plan_units(FaLaunch& L, uint32_t unit)
     L.nunits = units;
 }
 
+// The warps per CTA of a persistent launch that names none.  The build for
+// more warps holds a thread to fewer registers (65,536 / (32 x warps)); the
+// 32-warp one spills in the interpreter loop, and a lone warp is 16 % slower
+// in it.  So:
+// - 4K-bank carts: the smallest of 24, 28 and 32 that takes all units in one
+//   wave (20,000 mixed consoles x 4 frames: 6.4 ms at 24, 7.2 at 32; 135,500:
+//   17.2 at 28, two waves, 13.9 at 32).
+// - E0 / 3F carts: 24 (100,000 consoles x 4 frames: 63 ms; 72 at 28, 69 at 32).
+// - DPC, FE: CTAs of 4 (96 registers) while they can hold all units at once, up
+//   to 16 units per SM (16,000 DPC consoles x 2 frames: 1.51 against 1.68 ms,
+//   FE 2.58 against 2.87; at 21 per SM 3.64 against 2.99), then 24.
+// - carts of several kinds: CTAs of 4.  Every kind's core is in use on every
+//   SM, and fewer warps ask less of the instruction cache (100,000 consoles of
+//   plain, DPC, FE and 8 KB carts x 2 frames: 8.5 ms at 4, 11.6 at 16, 10.0 at
+//   24, 14.7 at 32; 600 consoles: 2.8, 3.0, 3.6, 4.1; nine carts, where the
+//   library leaves room for one CTA of 4 or 8 warps: 29 and 47 ms).
+static int auto_warps(int maps, uint32_t units, uint32_t lib, uint32_t slab, int sms)
+{
+    const uint32_t per = sms > 0 ? (units + (uint32_t)sms - 1u) / (uint32_t)sms : units;
+    if (maps == FA_MAPS_4K) return per <= 24u ? 24 : per <= 28u ? 28 : 32;
+    if (maps == FA_MAPS_SLICED) return 24;
+    if (maps == FA_MAPS_BOTH) return 4;
+    // What 4-warp CTAs keep resident: by shared memory (9 KB of tables and 1 KB
+    // of the system's per CTA), at most 20 warps of 96 registers.
+    const uint32_t ctas = FA_SMEM_PER_SM / (lib + 4u * slab + 10240u);
+    return per <= 16u && per <= 4u * ctas ? 4 : 24;
+}
+
 // The warp-granular layout of a launch: the ROM library, 32-instance work
 // units and the warps per CTA.  False when the library leaves no room for
 // block / 32 warp slabs (the launch is CTA-granular).
-static bool warp_layout(FaLaunch& L, int block, bool persistent, int* warps)
+static bool warp_layout(FaLaunch& L, int block, bool persistent, int sms, int* warps)
 {
     const uint32_t lib = plan_romlib(L);
     L.romlib_bytes = lib;
-    const uint32_t slab = fa_slab_words(fa_maps_of(L.g, L.ngroups)) * 32u * 4u;
+    const int maps = fa_maps_of(L.g, L.ngroups);
+    const uint32_t slab = fa_slab_words(maps) * 32u * 4u;
     const int fit = (int)((FA_SMEM_PER_CTA_MAX - (int)lib) / (int)slab);
     if (fit < block / 32) return false;
+    plan_units(L, 32u);
     int w = block / 32;
     if (persistent) {
-        // As many warps per CTA as shared memory allows (one CTA per SM), or
-        // fewer when a cap is set (the register budget per thread grows as
-        // 65536 / (32 x warps)).  A launch of sliced carts alone defaults to
-        // 24: at 32 warps its core is held to 64 registers and spills in the
-        // interpreter loop (three E0/3F carts: 2.31 against 2.13 M frames/s).
-        const int m = fa_maps_of(L.g, L.ngroups);
-        const int cap = L.cta_warps ? (int)L.cta_warps : (m == FA_MAPS_4K || m == FA_MAPS_BOTH) ? 32 : 24;
+        // As many as shared memory allows, up to the cap.
+        const int cap = L.cta_warps ? (int)L.cta_warps : auto_warps(maps, L.nunits, lib, slab, sms);
         static const int sizes[] = { 32, 28, 24, 16, 8, 4, 2 };
         for (int x : sizes)
             if (x <= fit && x <= cap) { w = x; break; }
     }
-    plan_units(L, 32u);
     *warps = w;
     return true;
 }
 
-cudaError_t fa_launch_run(const FaLaunch& L_in, int block, bool persistent, int sms, cudaStream_t s)
+// sms: the device's; launch_sms: the same, or 0 to prepare the launch only.
+static cudaError_t launch(const FaLaunch& L_in, int block, bool persistent, int sms, int launch_sms, cudaStream_t s)
 {
     FaLaunch L = L_in;
     L.wait_ns = fa_wait_limit_ns();
     const int maps = fa_maps_of(L.g, L.ngroups);                       // which cores the carts need
     int warps = 0;
-    if (warp_layout(L, block, persistent, &warps)) {
-        return maps == FA_MAPS_4K   ? FaCore<FA_MAPS_4K>::run_warps(warps, L, persistent, sms, s)
-             : maps == FA_MAPS_BOTH ? FaCore<FA_MAPS_BOTH>::run_warps(warps, L, persistent, sms, s)
-             : maps == FA_MAPS_DPC  ? FaCore<FA_MAPS_DPC>::run_warps(warps, L, persistent, sms, s)
-             : maps == FA_MAPS_FE   ? FaCore<FA_MAPS_FE>::run_warps(warps, L, persistent, sms, s)
-                                    : FaCore<FA_MAPS_SLICED>::run_warps(warps, L, persistent, sms, s);
+    if (warp_layout(L, block, persistent, sms, &warps)) {
+        return maps == FA_MAPS_4K   ? FaCore<FA_MAPS_4K>::run_warps(warps, L, persistent, launch_sms, s)
+             : maps == FA_MAPS_BOTH ? FaCore<FA_MAPS_BOTH>::run_warps(warps, L, persistent, launch_sms, s)
+             : maps == FA_MAPS_DPC  ? FaCore<FA_MAPS_DPC>::run_warps(warps, L, persistent, launch_sms, s)
+             : maps == FA_MAPS_FE   ? FaCore<FA_MAPS_FE>::run_warps(warps, L, persistent, launch_sms, s)
+                                    : FaCore<FA_MAPS_SLICED>::run_warps(warps, L, persistent, launch_sms, s);
     }
     // ROM library too large for shared memory: CTA-granular units that
     // re-stage one cart's ROM at a time.
     plan_units(L, (uint32_t)block);
-    return maps == FA_MAPS_4K   ? FaCore<FA_MAPS_4K>::run_block(block, L, persistent, sms, s)
-         : maps == FA_MAPS_BOTH ? FaCore<FA_MAPS_BOTH>::run_block(block, L, persistent, sms, s)
-         : maps == FA_MAPS_DPC  ? FaCore<FA_MAPS_DPC>::run_block(block, L, persistent, sms, s)
-         : maps == FA_MAPS_FE   ? FaCore<FA_MAPS_FE>::run_block(block, L, persistent, sms, s)
-                                : FaCore<FA_MAPS_SLICED>::run_block(block, L, persistent, sms, s);
+    return maps == FA_MAPS_4K   ? FaCore<FA_MAPS_4K>::run_block(block, L, persistent, launch_sms, s)
+         : maps == FA_MAPS_BOTH ? FaCore<FA_MAPS_BOTH>::run_block(block, L, persistent, launch_sms, s)
+         : maps == FA_MAPS_DPC  ? FaCore<FA_MAPS_DPC>::run_block(block, L, persistent, launch_sms, s)
+         : maps == FA_MAPS_FE   ? FaCore<FA_MAPS_FE>::run_block(block, L, persistent, launch_sms, s)
+                                : FaCore<FA_MAPS_SLICED>::run_block(block, L, persistent, launch_sms, s);
+}
+
+cudaError_t fa_launch_run(const FaLaunch& L, int block, bool persistent, int sms, cudaStream_t s)
+{
+    return launch(L, block, persistent, sms, sms, s);
 }
 
 bool fa_launch_warp_shape(const FaLaunch& L_in, int block, bool persistent, int sms, uint32_t* grid, uint32_t* warps,
@@ -111,7 +141,7 @@ bool fa_launch_warp_shape(const FaLaunch& L_in, int block, bool persistent, int 
     FaLaunch L = L_in;
     const int maps = fa_maps_of(L.g, L.ngroups);
     int w = 0;
-    if (!warp_layout(L, block, persistent, &w)) return false;
+    if (!warp_layout(L, block, persistent, sms, &w)) return false;
     *warps = (uint32_t)w;
     return maps == FA_MAPS_4K   ? FaCore<FA_MAPS_4K>::shape(w, L, persistent, sms, grid, per_sm)
          : maps == FA_MAPS_BOTH ? FaCore<FA_MAPS_BOTH>::shape(w, L, persistent, sms, grid, per_sm)
@@ -120,9 +150,9 @@ bool fa_launch_warp_shape(const FaLaunch& L_in, int block, bool persistent, int 
                                 : FaCore<FA_MAPS_SLICED>::shape(w, L, persistent, sms, grid, per_sm);
 }
 
-cudaError_t fa_launch_prepare(const FaLaunch& L, int block, bool persistent)
+cudaError_t fa_launch_prepare(const FaLaunch& L, int block, bool persistent, int sms)
 {
-    return fa_launch_run(L, block, persistent, 0, nullptr);
+    return launch(L, block, persistent, sms, 0, nullptr);
 }
 
 int fa_launch_occupancy(int block, uint32_t rom_bytes_max)

@@ -408,7 +408,7 @@ extern "C" int fa_pool_graph_create(fa_pool* p, const uint8_t* const* d_actions,
     // Warm the launch configuration cache outside the capture.
     FaLaunch L;
     build_launch(p, d_actions, (uint32_t)k, d_obs, 0, L);
-    FA_CUDA(fa_launch_prepare(L, p->block, p->persistent));
+    FA_CUDA(fa_launch_prepare(L, p->block, p->persistent, p->sms));
     rc = ensure_plan(p, L, (uint32_t)k);                                 // uploaded before the capture
     if (rc) return rc;
     const uint32_t* plan = L.first_wave;
