@@ -58,9 +58,13 @@ namespace fa {
 // or two 256-thread CTAs at 8).  Held to 80 registers for 24 resident warps,
 // the spills cost more than the extra warps gain: 2.15 against 3.92 M
 // frames/s on the render cart (113,664 consoles, one B200).  Uncapped,
-// ptxas takes 148, which a 16-warp CTA cannot launch with.
-template <int WARPS, bool SLICED>
-__global__ void __maxnreg__(128) fa_render_run(const __grid_constant__ FaRenderLaunch L)
+// ptxas takes 168, which a 16-warp CTA cannot launch with.  FEW, for consoles
+// that leave no more than 8 warps to an SM: those 168, without the spills
+// (4 frames, before and now: 64 consoles 21.8 and 19.0 ms, 18,944 22.3 and
+// 19.7, 28,416 25.5 and 23.7; at 12 warps to an SM, 56,832, it took 40.4
+// against 35.1, as the hardware deals the CTAs unevenly).
+template <int WARPS, bool SLICED, bool FEW>
+__global__ void __maxnreg__(FEW ? 168 : 128) fa_render_run(const __grid_constant__ FaRenderLaunch L)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t bar;
@@ -250,7 +254,7 @@ namespace {
 std::mutex g_rmu;
 std::map<std::pair<int, int>, bool> g_rcfg;   // (device, warps) whose smem limit was raised
 
-template <int WARPS, bool SLICED>
+template <int WARPS, bool SLICED, bool FEW>
 cudaError_t launch_render(const FaRenderLaunch& L, cudaStream_t s)
 {
     int dev = 0;
@@ -259,9 +263,9 @@ cudaError_t launch_render(const FaRenderLaunch& L, cudaStream_t s)
     const size_t smem = (size_t)L.nbanks * 4096u + (size_t)WARPS * FA_RSLAB_WORDS * 32u * 4u;
     {
         std::lock_guard<std::mutex> lk(g_rmu);
-        auto key = std::make_pair(dev, WARPS * 2 + (SLICED ? 1 : 0));
+        auto key = std::make_pair(dev, WARPS * 4 + (SLICED ? 1 : 0) + (FEW ? 2 : 0));
         if (g_rcfg.find(key) == g_rcfg.end()) {
-            e = cudaFuncSetAttribute(fa::fa_render_run<WARPS, SLICED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(fa::fa_render_run<WARPS, SLICED, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      32768 + WARPS * FA_RSLAB_WORDS * 32 * 4);
             if (e != cudaSuccess) return e;
             g_rcfg[key] = true;
@@ -272,13 +276,19 @@ cudaError_t launch_render(const FaRenderLaunch& L, cudaStream_t s)
     if (grid == 0) return cudaSuccess;
     FaRenderLaunch Lw = L;
     Lw.wait_ns = fa_wait_limit_ns();
-    fa::fa_render_run<WARPS, SLICED><<<grid, WARPS * 32, smem, s>>>(Lw);
+    fa::fa_render_run<WARPS, SLICED, FEW><<<grid, WARPS * 32, smem, s>>>(Lw);
     return cudaGetLastError();
+}
+
+template <int WARPS, bool FEW = false>
+cudaError_t launch_render_as(const FaRenderLaunch& L, cudaStream_t s)
+{
+    return fa_map_kind(L.hot_lo) != 0 ? launch_render<WARPS, true, FEW>(L, s)    // E0 / 3F carts
+                                      : launch_render<WARPS, false, FEW>(L, s);
 }
 
 cudaError_t launch_render_n(int warps, const FaRenderLaunch& L, cudaStream_t s)
 {
-    const bool sliced = fa_map_kind(L.hot_lo) != 0;                    // E0 / 3F carts
     // Few consoles spread over the SMs: CTAs of at most as many warps as every
     // SM gets (one 512-thread CTA took 16 warps to an SM while others idled:
     // 2,048 consoles x 4 frames 37 ms on 4 SMs, 18,944 x 2 frames 19 ms on 37).
@@ -288,12 +298,23 @@ cudaError_t launch_render_n(int warps, const FaRenderLaunch& L, cudaStream_t s)
     if (e != cudaSuccess) return e;
     const uint32_t units = (L.n + 31u) / 32u;
     while (warps > 1 && units / (uint32_t)sms < (uint32_t)warps) warps /= 2;
-    switch (warps) {
-    case 1: return sliced ? launch_render<1, true>(L, s) : launch_render<1, false>(L, s);
-    case 2: return sliced ? launch_render<2, true>(L, s) : launch_render<2, false>(L, s);
-    case 4: return sliced ? launch_render<4, true>(L, s) : launch_render<4, false>(L, s);
-    case 8: return sliced ? launch_render<8, true>(L, s) : launch_render<8, false>(L, s);
-    case 16: return sliced ? launch_render<16, true>(L, s) : launch_render<16, false>(L, s);
+    // The FEW build while two of its CTAs (of at most 4 warps) per SM hold
+    // every unit at once, or as many as a large ROM leaves room for (1 KB of
+    // shared memory per CTA is the system's, 9 KB are tables).
+    const uint32_t w4 = warps < 4 ? (uint32_t)warps : 4u;
+    const uint32_t ctas = FA_SMEM_PER_SM / (L.nbanks * 4096u + w4 * FA_RSLAB_WORDS * 128u + 10240u);
+    const uint32_t resident = w4 * ctas < 8u ? w4 * ctas : 8u;
+    if (units <= (uint32_t)sms * resident) {
+        switch (w4) {
+        case 1: return launch_render_as<1, true>(L, s);
+        case 2: return launch_render_as<2, true>(L, s);
+        case 4: return launch_render_as<4, true>(L, s);
+        }
+    }
+    switch (warps) {                                                   // 1 and 2: always above
+    case 4: return launch_render_as<4>(L, s);
+    case 8: return launch_render_as<8>(L, s);
+    case 16: return launch_render_as<16>(L, s);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -49,3 +49,21 @@ def test_picked_warps_give_the_same_results(family, per_sm, extra):
     for g in range(len(cs)):
         assert np.array_equal(got[0][0][g], got[1][0][g])
         assert np.array_equal(np.asarray(got[0][1][g]), np.asarray(got[1][1][g]))
+
+
+# Rendering consoles: the build for few consoles up to 8 warps per SM, and the
+# other one past that, at every CTA size.
+@pytest.mark.parametrize("n", [2 * SMS * 32, 4 * SMS * 32 - 1, 8 * SMS * 32, 8 * SMS * 32 + 1])
+def test_rendering_builds_agree(n):
+    c = carts.render_cart()
+    acts = carts.actions(seed=11, n=n, frames=1)
+    want = None
+    for warps in (16, 8, 4):
+        with fa.AtariRender(c.rom, n, cta_warps=warps) as r:
+            r.reset()
+            _, ram = r.step_multi(acts, 1, fb=False)
+            got = (np.asarray(ram).copy(), r.states(), r.rgba(0, 32).copy(), r.rgba(n - 32, 32).copy())
+        if want is None:
+            want = got
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b), f"{warps} warps"
