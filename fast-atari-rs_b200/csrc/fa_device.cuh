@@ -1473,7 +1473,7 @@ struct Emu {
     __device__ __forceinline__ uint32_t pia_span() const { return pia_span_of(tp & 0xFFFFu, tp >> 16, su & 0xFFFFu, su >> 16); }
     __device__ __forceinline__ uint2 pia_now() const { return pia_now_of(tp & 0xFFFFu, tp >> 16, su & 0xFFFFu, su >> 16, tlim); }
     // Fold the counted cycles in, run one exact call of n cycles (none for
-    // n = 0), and open the next window: one out-of-line copy.
+    // n = 0), and open the next window.
     __device__ __forceinline__ void pia_sync(uint32_t n)
     {
         const uint4 r = pia_sync_io(tp, su, tlim, n);
@@ -1746,10 +1746,12 @@ struct Emu {
     // whatever the opcode needs (always from this lane's RAM or the ROM
     // image), the frequent exceptions sit behind two tests, and the rest
     // (exec) apart.  Measured on one B200, before (a switch decoder with the
-    // time kept per instruction) and now: 165 and 109 warp instructions, 1,290
-    // and 470 cycles per guest instruction of a lone warp; a frame of one
-    // plain cart 3.45 and 1.30 ms; the mixed batch of 135,500 consoles x 4
-    // frames 23.2 and 16.0 ms; a frame of 50,000 divergence carts 7.1 and 3.1 ms.
+    // time kept per instruction) and now: 165 and 107 warp instructions, 1,290
+    // and 450 cycles per guest instruction of a lone warp; a frame of one
+    // plain cart 3.47 and 1.25 ms; the mixed batch of 135,500 consoles x 4
+    // frames 22.4 and 13.2 ms; a frame of 50,000 divergence carts 7.2 and 3.1 ms.
+    // Loading the next instruction's bytes and words while this one executes
+    // gained nothing (1.24 and 1.26 ms): the warp waits on the operations.
     template <class LOOK>
     __device__ __forceinline__ uint32_t run(uint32_t wait_key, LOOK look)
     {
