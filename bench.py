@@ -59,16 +59,16 @@ UNIT = "frames/s"
 # a warp run identical instances (fully converged), from the ncu capture in
 # profiles/fa_run_warps_converged_plain.md.  Used to express guest-instruction
 # throughput in warp-issue slots for the roofline.
-I_CONV = 165.5
+I_CONV = 110.8
 # DRAM bytes moved per instance-frame by fa_run on this workload, from the ncu
-# capture in profiles/fa_run_warps_mixed_batch_full.md (29.6 MB per 4-frame
+# capture in profiles/fa_run_warps_mixed_batch_full.md (29.5 MB per 4-frame
 # call of 135,500 instances).
-DRAM_BYTES_PER_INSTANCE_FRAME = 54.6
+DRAM_BYTES_PER_INSTANCE_FRAME = 54.4
 # The rendering kernel (fa_render_run) per rendered console-frame, from
 # the ncu capture in profiles/fa_render_run_render_cart.md: SASS
 # thread-instructions and DRAM bytes (framebuffer writes included).
-RENDER_THREAD_INST_PER_FRAME = 2.936e6   # smsp__thread_inst_executed / console-frames
-RENDER_DRAM_BYTES_PER_FRAME = 61_600     # (dram read + write) / console-frames
+RENDER_THREAD_INST_PER_FRAME = 2.234e6   # smsp__thread_inst_executed / console-frames
+RENDER_DRAM_BYTES_PER_FRAME = 60_400     # (dram read + write) / console-frames
 
 
 def load_pkg():

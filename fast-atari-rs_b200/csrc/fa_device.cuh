@@ -1237,7 +1237,6 @@ struct Emu {
 
     // ------------------------------------------------------------ flags
     __device__ __forceinline__ void set_nz(uint32_t v) { F = (F & 0xFFFF0000u) | v; }       // v: bytes 0 and 1
-    __device__ __forceinline__ void setc(uint32_t c) { F = (F & 0xFF00FFFFu) | (c << 16); }
     __device__ __forceinline__ void setv(uint32_t v) { F = (F & 0x00FFFFFFu) | (v << 24); }
     __device__ __forceinline__ uint32_t get_p() const
     {

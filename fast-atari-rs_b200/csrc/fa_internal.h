@@ -195,7 +195,7 @@ struct fa_handle {
     int block = 128;
     int sched = FA_SCHED_PC;
     bool persistent = false;
-    int cta_warps = 0;                 // persistent form: warps per CTA (0 = as many as fit)
+    int cta_warps = 0;                 // persistent form: warps per CTA (0: by the carts and units)
     uint32_t episode_frames = 0;
     unsigned long long last_instr = 0;
     unsigned long long last_slots = 0;

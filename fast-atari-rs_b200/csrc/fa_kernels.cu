@@ -61,15 +61,15 @@ static void plan_units(FaLaunch& L, uint32_t unit)
 // - 4K-bank carts: the smallest of 24, 28 and 32 that takes all units in one
 //   wave (20,000 mixed consoles x 4 frames: 6.4 ms at 24, 7.2 at 32; 135,500:
 //   17.2 at 28, two waves, 13.9 at 32).
-// - E0 / 3F carts: 24 (100,000 consoles x 4 frames: 63 ms; 72 at 28, 69 at 32).
+// - E0 / 3F carts: 24 (100,000 consoles x 4 frames: 62 ms; 72 at 28, 69 at 32).
 // - DPC, FE: CTAs of 4 (96 registers) while they can hold all units at once, up
-//   to 16 units per SM (16,000 DPC consoles x 2 frames: 1.51 against 1.68 ms,
-//   FE 2.58 against 2.87; at 21 per SM 3.64 against 2.99), then 24.
+//   to 16 units per SM (16,000 DPC consoles x 2 frames: 1.42 against 1.59 ms,
+//   FE 2.57 against 2.81; at 21 per SM 3.38 against 2.72), then 24.
 // - carts of several kinds: CTAs of 4.  Every kind's core is in use on every
 //   SM, and fewer warps ask less of the instruction cache (100,000 consoles of
-//   plain, DPC, FE and 8 KB carts x 2 frames: 8.5 ms at 4, 11.6 at 16, 10.0 at
-//   24, 14.7 at 32; 600 consoles: 2.8, 3.0, 3.6, 4.1; nine carts, where the
-//   library leaves room for one CTA of 4 or 8 warps: 29 and 47 ms).
+//   plain, DPC, FE and 8 KB carts x 2 frames: 7.7 ms at 4, 10.8 at 16, 8.9 at
+//   24, 14.5 at 32; 600 consoles: 2.8, 3.0, 3.6, 4.1; nine carts, where the
+//   library leaves room for one CTA of 4 or 8 warps: 28 and 44 ms).
 static int auto_warps(int maps, uint32_t units, uint32_t lib, uint32_t slab, int sms)
 {
     const uint32_t per = sms > 0 ? (units + (uint32_t)sms - 1u) / (uint32_t)sms : units;

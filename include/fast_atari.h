@@ -318,7 +318,7 @@ int fa_set_frame_numbers(fa_handle* h, const uint32_t* frame_no);
 int fa_set_launch(fa_handle* h, int block, int sched, int persistent);
 int fa_get_launch(const fa_handle* h, int* block, int* sched, int* persistent);
 
-/* Persistent form only: warps per CTA (0 = as many as shared memory fits;
+/* Persistent form only: warps per CTA (0 = by the carts and their number;
  * else 2, 4, 8, 16, 24, 28 or 32).  Fewer warps raise the register budget per
  * thread (65536 / (32 x warps)). */
 int fa_set_cta_warps(fa_handle* h, int warps);
