@@ -137,10 +137,12 @@ struct Runner {
 
     // Cycles until the frame loop must look again (Emu::dl): the timer's
     // window, the VSYNC budget or the frame's cycle cap.  The frame's elapsed
-    // cycles are its instruction cycles and its WSYNC waits (fcyc).
+    // cycles are its instruction cycles and its WSYNC waits (fcyc).  VSYNC may
+    // drop with the (smaller) cap already spent: none are left then.
     __device__ __forceinline__ uint32_t due() const
     {
-        return e.due((phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u - (e.cyc_acc + fcyc));
+        const uint32_t end = (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u, spent = e.cyc_acc + fcyc;
+        return e.due(end - (spent < end ? spent : end));
     }
 
     // One HeadlessAtari::run_one_cycle (src/atari.rs:601-614) after another
