@@ -34,8 +34,14 @@ struct RRunner {
         return true;
     }
     // The instruction cycles at which the frame loop must look: the VSYNC
-    // budget's or the frame cap's, less the frame's WSYNC waits.
-    __device__ __forceinline__ uint32_t due() const { return (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u - fcyc; }
+    // budget's or the frame cap's, less the frame's WSYNC waits.  VSYNC may
+    // drop with the (smaller) cap already spent: then at the next look, 0 if
+    // the waits alone spent it.
+    __device__ __forceinline__ uint32_t due() const
+    {
+        const uint32_t end = (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u;
+        return end - (fcyc < end ? fcyc : end);
+    }
 
     // After an instruction (ran), the frame-end checks of run_frame, then any
     // WSYNC wait it started, as a run_one_cycle of its own; until the frame
@@ -73,7 +79,7 @@ struct RRunner {
             // a per-cycle frame check would first fire: nothing else changes
             // from one cycle of the wait to the next.
             uint32_t n = (228u - e.clock + 2u) / 3u, lim = 1u;
-            if (phase || e.vsync_on()) lim = due() - e.cyc_acc;
+            if ((phase || e.vsync_on()) && e.cyc_acc < due()) lim = due() - e.cyc_acc;
             n = n < lim ? n : lim;
             e.rcycles(n);
             fcyc += n;

@@ -13,6 +13,7 @@ import pytest
 import oracle
 from fa_pkg import carts, fa
 from test_edge_programs import KINDS, program, states
+from test_gpu_render import check
 from test_host_sim import assert_same, run_both, sim  # noqa: F401  (the fixture)
 
 ORG = 0xFC00                       # in the window that no scheme switches (E0, 3F), the same in every bank
@@ -101,6 +102,31 @@ def test_random_programs_that_start_in_vsync(sim, kind, seed):  # noqa: F811
     assert_same(got, ref, f"{kind} program {seed}")
 
 
+RENDERED = ["4k", "8k", "32k", "e0", "3f"]
+
+
+@pytest.mark.parametrize("kind", RENDERED)
+def test_vsync_held_past_the_frame_cap_on_the_rendering_console(sim, kind):  # noqa: F811
+    """Its frame loop looks at instruction cycles and counts a WSYNC wait cycle by cycle."""
+    size, code = KINDS[kind]
+    n, calls, k = 1, 2, 1
+    acts = np.stack([carts.actions(seed=50 + i, n=n, frames=k) for i in range(calls)])
+    for delay in ("loop", "wsync"):
+        for drop in DROPS:
+            for after in AFTER:
+                rom = hold_rom(size, delay, drop, after)
+                r = np.frombuffer(rom, np.uint8).copy()
+                fb, ram = np.zeros((n, 192, 160), np.uint8), np.zeros((n, 128), np.uint8)
+                st = np.zeros(n, fa.STATE_DTYPE)
+                with scheme_of(rom, code, on_host(sim)):
+                    assert sim.hs_render(r.ctypes.data, len(r), n, acts.ctypes.data, calls, k, fb.ctypes.data,
+                                         st.ctypes.data, ram.ctypes.data) >= 0
+                    consoles = oracle.render_reset(rom, n)
+                    for i in range(calls):
+                        oracle.render_steps(consoles, acts[i])
+                check(fb, ram, st, consoles, f"{kind}, {delay}, {drop}, {after}")
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", KINDS)
 def test_vsync_held_past_the_frame_cap_on_the_gpu(kind):
@@ -120,3 +146,22 @@ def test_vsync_held_past_the_frame_cap_on_the_gpu(kind):
                 got = g.download_states()
             oracle.run_batch(rom, ref, acts, k)
             assert_same(got, ref, f"{kind}, {delay}, {drop}, {after}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", RENDERED)
+def test_vsync_held_past_the_frame_cap_on_the_rendering_console_on_the_gpu(kind):
+    if fa.device_count() < 1:
+        pytest.skip("no CUDA device")
+    size, code = KINDS[kind]
+    n, k = 33, 2
+    acts = carts.actions(seed=50, n=n, frames=k)
+    for delay, drop, after in [("wsync", "store", "jump"), ("wsync", "brk", "wait"), ("loop", "store", "illegal")]:
+        rom = hold_rom(size, delay, drop, after)
+        with scheme_of(rom, code, lambda r, c: fa.set_rom_scheme(r, c if c >= 0 else "auto")):
+            consoles = oracle.render_reset(rom, n)
+            oracle.render_steps(consoles, acts)
+            with fa.AtariRender(rom, n) as g:
+                g.reset()
+                fb, ram = g.step_multi(acts, k)
+                check(fb, ram, g.states(), consoles, f"{kind}, {delay}, {drop}, {after}")
