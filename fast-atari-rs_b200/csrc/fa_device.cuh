@@ -1771,7 +1771,7 @@ struct Emu {
             const uint32_t b1 = lds8(q + 1), b2 = lds8(q + 2);
             OpWord w = ldw(tab, op);
             const uint32_t f = w.ix;
-            const uint32_t pc1 = pc + high<!RENDER>(tab, op, H_LEN, w.rd);            // past $FFFF: not ok, and exec() masks it
+            const uint32_t pc1 = pc + high<!RENDER>(tab, op, H_LEN, w.rd);            // may pass $FFFF: not ok then
             uint32_t base = __byte_perm(b1, b2, w.bs);
             n = high<!RENDER>(tab, op, H_CYC, w.rs);
             if (!ok | ((f & T_CTRL) != 0u)) {
@@ -1956,6 +1956,7 @@ struct Emu {
                 if (!look(n)) break;
             }
         } while ((kb | pc) < wait_key);
+        pc &= 0xFFFFu;                                                // an instruction may have left it past $FFFF
         return 1u;
     }
 
