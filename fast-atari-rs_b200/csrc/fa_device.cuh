@@ -1956,7 +1956,6 @@ struct Emu {
                 if (!look(n)) break;
             }
         } while ((kb | pc) < wait_key);
-        pc &= 0xFFFFu;                                                // an instruction may have left it past $FFFF
         return 1u;
     }
 
@@ -2354,7 +2353,8 @@ struct Emu {
     __device__ __forceinline__ void store_hot(uint32_t* col, uint32_t stride) const
     {
         col[R_AXYS * stride] = R;
-        col[R_PC * stride] = pc | (get_p() << 16) | ((bank >> 12) << 24);
+        // pc is masked where an instruction starts: the last one may have left it past $FFFF.
+        col[R_PC * stride] = (pc & 0xFFFFu) | (get_p() << 16) | ((bank >> 12) << 24);
         col[R_PIA0 * stride] = (ports & 0xFFFFu) | ((pins & 0xFFu) << 16) | (((ports >> 16) & 0xFFu) << 24);
         col[R_PIA1 * stride] = (ports >> 24) | (((pins >> 8) & 0xFFu) << 8) | ((su >> 16) << 16) | (((tw >> 18) & 1u) << 24);
         const uint2 t = RENDER ? make_uint2(tp & 0xFFFFu, tp >> 16) : pia_now();

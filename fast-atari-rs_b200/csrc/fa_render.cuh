@@ -34,14 +34,9 @@ struct RRunner {
         return true;
     }
     // The instruction cycles at which the frame loop must look: the VSYNC
-    // budget's or the frame cap's, less the frame's WSYNC waits.  VSYNC may
-    // drop with the (smaller) cap already spent: then at the next look, 0 if
-    // the waits alone spent it.
-    __device__ __forceinline__ uint32_t due() const
-    {
-        const uint32_t end = (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u;
-        return end - (fcyc < end ? fcyc : end);
-    }
+    // budget's or the frame cap's, less the frame's WSYNC waits; after
+    // attend's checks above cyc_acc.
+    __device__ __forceinline__ uint32_t due() const { return (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u - fcyc; }
 
     // After an instruction (ran), the frame-end checks of run_frame, then any
     // WSYNC wait it started, as a run_one_cycle of its own; until the frame
@@ -59,7 +54,13 @@ struct RRunner {
                         active = false;
                         return;
                     }
-                    if (!e.vsync_on()) phase = 1u;
+                    if (!e.vsync_on()) {
+                        // VSYNC may drop with the (smaller) cap more than
+                        // spent: spent to the cycle, it ends the frame after
+                        // the next instruction or cycle of a wait too.
+                        phase = 1u;
+                        if (fc > FA_FRAME_CYCLE_CAP) fcyc = FA_FRAME_CYCLE_CAP - e.cyc_acc;
+                    }
                 } else {
                     const bool cap = fc > FA_FRAME_CYCLE_CAP;
                     if (cap || e.vsync_on()) {
@@ -79,7 +80,7 @@ struct RRunner {
             // a per-cycle frame check would first fire: nothing else changes
             // from one cycle of the wait to the next.
             uint32_t n = (228u - e.clock + 2u) / 3u, lim = 1u;
-            if ((phase || e.vsync_on()) && e.cyc_acc < due()) lim = due() - e.cyc_acc;
+            if (phase || e.vsync_on()) lim = due() - e.cyc_acc;
             n = n < lim ? n : lim;
             e.rcycles(n);
             fcyc += n;
@@ -90,10 +91,10 @@ struct RRunner {
 
     __device__ __forceinline__ uint32_t key(uint32_t sched) const
     {
-        if (sched != FA_SCHED_LINE) return e.kb | e.pc;
-        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | e.pc;
+        if (sched != FA_SCHED_LINE) return e.kb | (e.pc & 0xFFFFu);
+        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | (e.pc & 0xFFFFu);
     }
-    __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | e.pc; }
+    __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | (e.pc & 0xFFFFu); }
     // Instructions of this lane up to one that may leave the lanes of its
     // group at different pcs, that reaches a waiting lane's key, or after
     // which the frame loop must look (and the WSYNC waits it started).

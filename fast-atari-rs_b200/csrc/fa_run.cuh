@@ -137,12 +137,11 @@ struct Runner {
 
     // Cycles until the frame loop must look again (Emu::dl): the timer's
     // window, the VSYNC budget or the frame's cycle cap.  The frame's elapsed
-    // cycles are its instruction cycles and its WSYNC waits (fcyc).  VSYNC may
-    // drop with the (smaller) cap already spent: none are left then.
+    // cycles are its instruction cycles and its WSYNC waits (fcyc): none at its
+    // start, no more than the cap after a wait taken in one piece.
     __device__ __forceinline__ uint32_t due() const
     {
-        const uint32_t end = (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u, spent = e.cyc_acc + fcyc;
-        return e.due(end - (spent < end ? spent : end));
+        return e.due((phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u - (e.cyc_acc + fcyc));
     }
 
     // One HeadlessAtari::run_one_cycle (src/atari.rs:601-614) after another
@@ -205,7 +204,10 @@ struct Runner {
             if (n == 0u) break;
             fcyc += n;
         }
-        e.dl = due();
+        // due(), but VSYNC may have dropped with the (smaller) cap spent: none
+        // are left then, and the next instruction ends the frame.
+        const uint32_t end = (phase ? FA_FRAME_CYCLE_CAP : FA_VSYNC_BUDGET) + 1u, spent = e.cyc_acc + fcyc;
+        e.dl = e.due(end - (spent < end ? spent : end));
     }
 
     // Instructions of this lane up to one that may leave the lanes of its
@@ -233,12 +235,12 @@ struct Runner {
     // (FA_SCHED_LINE), then pc.
     __device__ __forceinline__ uint32_t key(uint32_t sched)
     {
-        if (sched != FA_SCHED_LINE) return e.kb | e.pc;
+        if (sched != FA_SCHED_LINE) return e.kb | (e.pc & 0xFFFFu);
         e.sync();
-        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | e.pc;
+        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | (e.pc & 0xFFFFu);
     }
     // Where the lane is: pc, bank and bank-switch count.
-    __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | e.pc; }
+    __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | (e.pc & 0xFFFFu); }
     __device__ __forceinline__ void iterate() { burst(0xFFFFFFFFu); }
 };
 
