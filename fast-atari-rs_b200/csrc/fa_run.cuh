@@ -278,7 +278,9 @@ __device__ __forceinline__ uint32_t run_lanes(RUNNER& r, uint32_t sched)
             if (!__any_sync(FULL, act)) break;
             const uint32_t key = act ? r.key(sched) : 0xFFFFFFFFu;
             const uint32_t mk = __reduce_min_sync(FULL, key);
-            lead = __ffs(__ballot_sync(FULL, key == mk)) - 1u;
+            // A lane that does not run has the greatest key, which one that
+            // does may have too (frame 127 or later, 511 hotspot accesses, $FFFF).
+            lead = __ffs(__ballot_sync(FULL, act && key == mk)) - 1u;
             // Every lane takes part in the full-mask shuffle, so it is not
             // folded into a short-circuit condition.
             const uint32_t lpcb = __shfl_sync(FULL, pcb, lead);
