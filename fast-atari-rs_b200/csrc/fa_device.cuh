@@ -2330,9 +2330,7 @@ struct Emu {
     {
         uint32_t w;
         R = col[R_AXYS * stride];
-        w = col[R_PC * stride];    pc = w & 0xFFFF; set_p((w >> 16) & 0xFF);
-        // 4K-bank carts: within the image, whatever the row holds (its loads are unconditional).
-        bank = ((w >> 24) & (SLICED ? 7u : nbanks - 1u)) << 12;
+        w = col[R_PC * stride];    pc = w & 0xFFFF; set_p((w >> 16) & 0xFF); bank = (w >> 24) << 12;
         cyc_acc = 0; el = 0; tl = 0; plag = 0;
         const uint32_t p0 = col[R_PIA0 * stride];                  // pa_out pa_ddr pa_in pb_out
         const uint32_t p1 = col[R_PIA1 * stride];                  // pb_ddr pb_in uf pdump

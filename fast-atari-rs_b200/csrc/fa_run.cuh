@@ -352,6 +352,8 @@ __device__ __forceinline__ void run_unit_as(const FaGroup& G, uint32_t first, ui
     if (valid) {
         r.e.load_ram(col, G.stride);
         r.e.load_hot(col, G.stride);
+        // Within the image, whatever the row holds: its loads are unconditional.
+        if constexpr (!SLICED) r.e.bank &= (G.nbanks - 1u) << 12;
         if constexpr (DPC) r.e.load_dpc();
         if (G.k > 0) r.active = r.begin_frame();
     }

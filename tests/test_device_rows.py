@@ -5,11 +5,12 @@ import pytest
 
 import oracle
 from fa_pkg import carts
-from test_host_sim import assert_same, run_both, sim  # noqa: F401  (the fixture)
+from test_host_sim import assert_same
+from test_host_warp import run_warps, warp  # noqa: F401  (the fixture)
 
 
 @pytest.mark.parametrize("size", [4096, 8192, 16384, 32768])
-def test_bank_outside_the_image(sim, size):  # noqa: F811
+def test_bank_outside_the_image(warp, size):  # noqa: F811
     """A 4K-bank cart's bank byte selects a bank of the image whatever it holds: its number modulo the banks."""
     rng = np.random.default_rng(size)
     nbanks = size // 4096
@@ -23,7 +24,7 @@ def test_bank_outside_the_image(sim, size):  # noqa: F811
     tame = wild.copy()
     wild["bank"], tame["bank"] = banks, banks % nbanks
     acts = carts.actions(seed=4, n=len(banks), frames=2)
-    _, ref = run_both(sim, rom, tame, acts, 2)             # the oracle takes no bank outside the image
-    r = np.frombuffer(rom, np.uint8).copy()
-    assert sim.hs_run(r.ctypes.data, len(r), wild.ctypes.data, len(wild), acts.ctypes.data, 2) >= 0
-    assert_same(wild, ref, f"{size}-byte cart")
+    got = run_warps(warp, rom, wild, acts, 2, "lane", 20_000_000)
+    ref = tame.copy()                                      # the oracle takes no bank outside the image
+    oracle.run_batch(rom, ref, acts, 2)
+    assert_same(got, ref, f"{size}-byte cart")
