@@ -1248,10 +1248,11 @@ struct Emu {
         pd = (v & F_D) ? T_UV : 0u;
         F = ((v & F_Z) ? 0u : 1u) | ((v & F_N) << 8) | ((v & F_C) << 16) | ((v & F_V) << 25);
     }
-    // One more hotspot access this frame (a scheduling key only, saturating).
+    // One more hotspot access this frame (a scheduling key only, saturating;
+    // at 510, so that no key is all ones).
     __device__ __forceinline__ void bump()
     {
-        if ((kb & 0x01FF0000u) != 0x01FF0000u) kb += 0x10000u;
+        if ((kb & 0x01FF0000u) != 0x01FE0000u) kb += 0x10000u;
     }
 
     // ------------------------------------------------------------ bank switching

@@ -92,7 +92,7 @@ struct RRunner {
     __device__ __forceinline__ uint32_t key(uint32_t sched) const
     {
         if (sched != FA_SCHED_LINE) return e.kb | (e.pc & 0xFFFFu);
-        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | (e.pc & 0xFFFFu);
+        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FEu ? e.scanline : 0x1FEu) << 16) | (e.pc & 0xFFFFu);
     }
     __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | (e.pc & 0xFFFFu); }
     // Instructions of this lane up to one that may leave the lanes of its

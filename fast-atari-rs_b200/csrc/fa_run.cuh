@@ -232,12 +232,13 @@ struct Runner {
     // then the hotspot accesses of this frame (FA_SCHED_PC; the same code
     // address in two banks is two program points, and a lane that has
     // switched banks once more is ahead whatever its pc) or the scanline
-    // (FA_SCHED_LINE), then pc.
+    // (FA_SCHED_LINE), then pc.  Never all ones, which stands for a lane that
+    // does not run: the middle field ends at 510.
     __device__ __forceinline__ uint32_t key(uint32_t sched)
     {
         if (sched != FA_SCHED_LINE) return e.kb | (e.pc & 0xFFFFu);
         e.sync();
-        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FFu ? e.scanline : 0x1FFu) << 16) | (e.pc & 0xFFFFu);
+        return (e.kb & 0xFE000000u) | ((e.scanline < 0x1FEu ? e.scanline : 0x1FEu) << 16) | (e.pc & 0xFFFFu);
     }
     // Where the lane is: pc, bank and bank-switch count.
     __device__ __forceinline__ uint32_t place() const { return (e.kb & 0x01FF0000u) | (e.bank << 13) | (e.pc & 0xFFFFu); }
@@ -278,9 +279,7 @@ __device__ __forceinline__ uint32_t run_lanes(RUNNER& r, uint32_t sched)
             if (!__any_sync(FULL, act)) break;
             const uint32_t key = act ? r.key(sched) : 0xFFFFFFFFu;
             const uint32_t mk = __reduce_min_sync(FULL, key);
-            // A lane that does not run has the greatest key, which one that
-            // does may have too (frame 127 or later, 511 hotspot accesses, $FFFF).
-            lead = __ffs(__ballot_sync(FULL, act && key == mk)) - 1u;
+            lead = __ffs(__ballot_sync(FULL, key == mk)) - 1u;
             // Every lane takes part in the full-mask shuffle, so it is not
             // folded into a short-circuit condition.
             const uint32_t lpcb = __shfl_sync(FULL, pcb, lead);
