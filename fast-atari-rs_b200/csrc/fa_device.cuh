@@ -2014,11 +2014,22 @@ struct Emu {
         }
     }
 
-    // Whether the lanes running this branch together part on it.
+    // Whether the lanes running this branch together part on it.  The lanes
+    // that read a mask are those it names, and each goes on to the vote with
+    // it: one statement, so that nothing comes between and no lane of the mask
+    // stays away.  Which lanes run together here is not promised: how soon the
+    // scheduler is asked depends on it, never a result.
     __device__ __forceinline__ static bool parted(bool tk)
     {
 #ifdef __CUDA_ARCH__
-        const uint32_t am = __activemask(), tb = __ballot_sync(am, tk);
+        uint32_t am, tb;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.u32 p, %2, 0;\n\t"
+            "activemask.b32 %0;\n\t"
+            "vote.sync.ballot.b32 %1, p, %0;\n\t}"
+            : "=&r"(am), "=r"(tb)
+            : "r"((uint32_t)tk));
         return (tb != 0u) & (tb != am);
 #else
         (void)tk;
