@@ -2,8 +2,8 @@
 //
 // For one ROM and an instance count, measures (CUDA events on the handle's
 // stream) frames/s over a staged sweep: the warp scheduling policy, then the
-// launch shape (persistent CTAs of 8..32 warps, i.e. register caps of
-// 256..64 registers per thread, or the plain form with 64..512-thread CTAs),
+// launch shape (persistent CTAs of the launch's own choice or of 8, 16 or 24
+// warps, or the plain form with 64..512-thread CTAs),
 // then the frames per launch K.  Every configuration produces identical
 // results; only the time differs.  The best record is what a pool or handle
 // should use for the cart, and its cost per instance-frame is the pool's

@@ -1,10 +1,14 @@
 // fa_device.cuh — the per-thread Atari 2600 emulator for sm_100a.
 //
-// One thread emulates one console.  Its hot state lives in registers; its
-// 128-byte PIA RAM and the TIA registers that change only on a write live in
-// shared memory, interleaved by thread in 32-bit words (byte o of thread t is
-// at word (o/4)*BLOCK + t), so lanes touching any offsets hit bank t%32 and
-// never conflict.  ROM banks sit in shared memory, staged once per block.
+// One thread emulates one console.  Its hot state lives in registers, its
+// 128-byte PIA RAM in shared memory.  Headless consoles interleave the RAM by
+// byte (byte o of thread t at o * BLOCK + t): one multiply to reach, up to
+// four lanes at different offsets on a bank.  Their TIA registers that change
+// only on a write stay in the HBM state rows; the DPC core's registers come
+// into shared memory while a unit runs.  Rendering consoles keep RAM and
+// graphics registers there, interleaved by 32-bit word (byte o of lane t in
+// word (o/4)*32 + t), so that no two lanes meet on a bank.  ROM banks sit in
+// shared memory, staged once per block.
 //
 // Semantics are those of the reference CPU emulator (RPP1011/fast-atari-rs):
 //   src/cpu.rs            6502 step, including every phantom access whose
@@ -2257,9 +2261,9 @@ struct Emu {
     // ------------------------------------------------------------ rendering console
     // Used only by RENDER instantiations.  The pixel-accurate Tia of the
     // reference's rendering console (src/tia.rs) and Pia::tick run out of
-    // line (render_cycles / render_tia_ticks / render_io_read / render_write_cycle,
-    // below), on the state they touch passed by value: one copy of the pixel
-    // pipeline however many bus-access sites the interpreter has.
+    // line (render_clocks, render_write, render_read, render_observe and
+    // r_pia_ticks, above), on the state they touch passed by value: one copy of
+    // the pixel pipeline however many bus-access sites the interpreter has.
     uint32_t done;            // instruction cycles of the frame (cyc_acc) at which the frame loop must look
     uint32_t lag;             // CPU cycles not yet given to the TIA; within an instruction, up to its start
                              // (negative: they have reached cycle -lag of it)

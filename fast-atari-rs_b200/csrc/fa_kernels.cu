@@ -30,8 +30,7 @@ __global__ void fa_broadcast(uint32_t* state, uint32_t stride, uint32_t n, const
 }  // namespace fa
 
 // ------------------------------------------------------------------ host launchers
-// Lay out the ROM library (one copy per distinct ROM buffer) and the work
-// units; returns the library size, or 0 if it cannot fit beside one warp slab.
+// Lay out the ROM library (one copy per distinct ROM buffer); returns its size.
 static uint32_t plan_romlib(FaLaunch& L)
 {
     uint32_t bytes = 0;
@@ -69,7 +68,12 @@ static void plan_units(FaLaunch& L, uint32_t unit)
 //   SM, and fewer warps ask less of the instruction cache (100,000 consoles of
 //   plain, DPC, FE and 8 KB carts x 2 frames: 7.7 ms at 4, 10.8 at 16, 8.9 at
 //   24, 14.5 at 32; 600 consoles: 2.8, 3.0, 3.6, 4.1; nine carts, where the
-//   library leaves room for one CTA of 4 or 8 warps: 28 and 44 ms).
+//   library leaves room for one CTA of 4 or 8 warps: 28 and 44 ms).  Not the
+//   best everywhere: from a library of 83 KB on one CTA of 4 is all that an SM
+//   holds, which costs once there is more than a wave of them (with an E0
+//   cart, x 2 frames, at 4, 8, 16 and 24 warps: 100,000 consoles and 32 KB of
+//   library 16.6, 18.3, 17.9, 21.4 ms, 84 KB 28.3, 18.3, 17.5, 21.3, 124 KB
+//   20.4, 17.9, 19.7, 20.3; 20,000 consoles and 84 KB 11.1, 11.0, 11.6, 12.8).
 static int auto_warps(int maps, uint32_t units, uint32_t lib, uint32_t slab, int sms)
 {
     const uint32_t per = sms > 0 ? (units + (uint32_t)sms - 1u) / (uint32_t)sms : units;
@@ -120,8 +124,10 @@ static cudaError_t launch(const FaLaunch& L_in, int block, bool persistent, int 
              : maps == FA_MAPS_FE   ? FaCore<FA_MAPS_FE>::run_warps(warps, L, persistent, launch_sms, s)
                                     : FaCore<FA_MAPS_SLICED>::run_warps(warps, L, persistent, launch_sms, s);
     }
-    // ROM library too large for shared memory: CTA-granular units that
-    // re-stage one cart's ROM at a time.
+    // ROM library too large for shared memory (with blocks of 128
+    // over 200 KB, over 196 with DPC carts or several kinds):
+    // CTA-granular units that re-stage one cart's ROM at a time.  100,000 4K-bank
+    // consoles x 2 frames: 17.0 ms with 196 KB (resident), 7.3 with 204 (re-staged).
     plan_units(L, (uint32_t)block);
     return maps == FA_MAPS_4K   ? FaCore<FA_MAPS_4K>::run_block(block, L, persistent, launch_sms, s)
          : maps == FA_MAPS_BOTH ? FaCore<FA_MAPS_BOTH>::run_block(block, L, persistent, launch_sms, s)

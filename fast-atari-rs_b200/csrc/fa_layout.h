@@ -53,8 +53,8 @@ enum : uint32_t {
     R_TIA2   = FA_PRIV_WORDS + 10,  // inpt4 | inpt5<<8 | paddle0<<16 | paddle1<<24
     R_FRAME  = FA_PRIV_WORDS + 11,  // frame_no
     R_STATUS = FA_PRIV_WORDS + 12,  // run_status
-    // DPC registers (FA_SCHEME_DPC carts only; the device touches them only
-    // on a DPC register access, in place in HBM).
+    // DPC registers (FA_SCHEME_DPC carts only; in the console's shared-memory
+    // slab while a unit runs, Emu::load_dpc and store_dpc).
     R_DPC_CNT = FA_PRIV_WORDS + 13, // 4 rows: counter 2r | counter 2r+1 << 16
     R_DPC_TOP = FA_PRIV_WORDS + 17, // 2 rows: top 4r..4r+3, one per byte
     R_DPC_BOT = FA_PRIV_WORDS + 19, // 2 rows: bottom 4r..4r+3
