@@ -36,7 +36,7 @@ constexpr uint32_t FA_REQ_FAILED = 0x80000000u;   // bit of a request's unit cou
 // by core, and one such CTA is resident, without spills.  Held to 64 registers
 // for 32 warps, 60 requests took 33 against 23-28 ms, the load at 3 M frames/s
 // a median of 11.3 against 10.5 ms, and the peak was the same.  60 requests in
-// CTAs of 4, 8 and 16 warps, on one box: 18.2, 18.9 and 21.3 ms.
+// CTAs of 4, 8 and 16 warps, one B200: 18.2, 18.9 and 21.3 ms.
 template <int WARPS, int MAPS>
 __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) fa_serve(const __grid_constant__ FaServeLaunch L)
 {
